@@ -233,7 +233,7 @@ def run_micsa(a, dist):
     stream = torch.cuda.ExternalStream(ctx.stream(), device=dev)
     attempts = float(L ** 3) * nr * ns * nc
     # ---- device-resident throughput: the K steps in one call (graph replays,
-    # or multi-iteration launches of the resident kernel at L <= 16)
+    # or multi-iteration launches of the resident kernel at L <= 32)
     ctx.iterate(a.warmup)
     ctx.synchronize()
     dist.barrier()

@@ -28,7 +28,9 @@
  *                        micsa_create (meanings at micsa_tuning_report)
  *   MICSA_TUNE_CACHE=0   time every context instead of reusing the process's
  *                        choice for its shape
- *   MICSA_RESIDENT=0     keep L <= 16 on the per-half-sweep kernels
+ *   MICSA_RESIDENT=0     keep L <= 32 on the per-half-sweep kernels
+ *   MICSA_RESIDENT_CTAS=c  blocks per cluster of the resident kernel (1, 2, 4 or 8
+ *                        where the shape has that size), for calls of any length
  *   MICSA_PDL=0          plain launches instead of programmatic dependent launch
  *   MICSA_REFRESH_WPS=n  segment length of the GPU demon refresh, in words
  *   MICSA_REFRESH_OCC=1  the refresh kernel without its register budget
@@ -156,11 +158,13 @@ int micsa_refresh_commit(micsa_ctx *ctx);
 int micsa_monte_carlo(micsa_ctx *ctx, int flag, const uint32_t *te,
                       const uint32_t *keys);
 /* n microcanonical iterations back to back (flag = 1 each), replayed from a
- * CUDA graph of one iteration; at L = 8 and 16 (where a sample's state fits
- * in one block's shared memory) up to 1024 whole iterations per launch of a
- * shared-memory-resident kernel instead (MICSA_RESIDENT=0 in the environment
- * at micsa_create turns that off).  Results are identical either way.
- * Asynchronous. */
+ * CUDA graph of one iteration; at L = 8, 16, 24 and 32 (where one replica
+ * word of a sample fits the shared memory of a block or of a cluster of up to
+ * 8) up to 1024 whole iterations per launch of a shared-memory-resident
+ * kernel instead, when the call is long enough to pay for copying the state
+ * in and out (MICSA_RESIDENT=0 in the environment at micsa_create turns that
+ * off, as does a pinned sweep shape above L = 16).  Results are identical
+ * either way.  Asynchronous. */
 int micsa_iterate(micsa_ctx *ctx, int64_t n);
 
 /* Measurements of every sample at the current state (Measure_Energy_Spins
@@ -381,7 +385,7 @@ int micsa_server_destroy(micsa_server *sv);
  * it before any state is uploaded (with state present the defaults are
  * kept; MICSA_MULTI_ZC=z pins the slab depth where it divides L).  The
  * choice is kept per process for the same list of shapes.  At most 16
- * contexts.  A context whose samples fit one block's shared memory (L <= 16,
+ * contexts.  A context whose samples fit shared memory (L <= 32,
  * the resident kernel of micsa_iterate) keeps that kernel, issued on its own
  * stream beside the mixed launch (MICSA_MULTI_RESIDENT=0 puts it in the
  * launch too); a launch carries one or more iterations (timed: 1, 4 or 16;

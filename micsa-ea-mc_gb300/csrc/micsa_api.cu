@@ -48,7 +48,9 @@ struct micsa_ctx {
   std::vector<cudaGraphExec_t> rem_exec;
   std::vector<int64_t> rem_launches;
   int64_t launches = 0;
-  int resident = 0;        /* small lattice: iterations run in shared memory */
+  int resident = 0;        /* small lattice: iterations run in shared memory, by clusters of
+                              this many blocks per sample and replica word (0: not) */
+  int64_t resident_min = 1; /* calls of fewer iterations run half-sweep by half-sweep */
   int split = 0;           /* k > 0: half-sweep launches per group of k samples, group-major
                               (a smaller L2 working set); 0: all samples per launch */
   micsa_tma tma = {};      /* tensor maps of the demon arrays (staged sweep) */
@@ -777,13 +779,17 @@ int micsa_create(const micsa_config *cfg, micsa_ctx **out) {
   MICSA_CK_CREATE(cudaMemsetAsync(ctx->dem1, 0, 4 * s.dem_w, ctx->stream));
   MICSA_CK_CREATE(cudaStreamSynchronize(ctx->stream));
   {
-    /* MICSA_RESIDENT=0 keeps small lattices on the per-half-sweep kernels */
-    const char *er = getenv("MICSA_RESIDENT");
-    const size_t need = micsa_resident_smem(cfg->L, cfg->nc);
+    /* MICSA_RESIDENT=0 keeps small lattices on the per-half-sweep kernels, as
+     * does a pinned sweep shape above L = 16; MICSA_RESIDENT_CTAS=c pins the
+     * cluster size */
+    const char *er = getenv("MICSA_RESIDENT"), *ec = getenv("MICSA_RESIDENT_CTAS");
     int optin = 0;
     MICSA_CK_CREATE(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                            cfg->device));
-    ctx->resident = need > 0 && need <= (size_t)optin && !(er && !strcmp(er, "0"));
+    if (!(er && !strcmp(er, "0")) && (cfg->L <= 16 || !getenv("MICSA_SWEEP_ZC")))
+      MICSA_CK_CREATE(micsa_resident_shape(cfg->L, cfg->nc, g.W, cfg->nsamples, optin,
+                                           ec ? atoi(ec) : 0, &ctx->resident,
+                                           &ctx->resident_min));
   }
   MICSA_CK_CREATE(micsa_make_tma(ctx->g, ctx->dem0, ctx->dem1, &ctx->tma));
   if ((rc = autotune(ctx)) != MICSA_OK) {
@@ -1237,7 +1243,8 @@ int micsa_iterate(micsa_ctx *ctx, int64_t n) {
    * carry several per launch); the remainder k < fit runs as one launch of k
    * iterations, from a graph made on first use */
   const int unit = ctx->g.flow && ctx->g.fit > 1 ? ctx->g.fit : 1;
-  if (!ctx->graph_exec && !ctx->resident &&
+  const bool resident = ctx->resident && (n >= ctx->resident_min || n == 0);
+  if (!ctx->graph_exec && !resident &&
       (rc = capture_iterations(ctx, unit, &ctx->graph, &ctx->graph_exec, &ctx->graph_launches)))
     return rc;
   const int left = unit > 1 ? (int)(n % unit) : 0;
@@ -1252,11 +1259,11 @@ int micsa_iterate(micsa_ctx *ctx, int64_t n) {
                                  &ctx->rem_launches[left])))
       return rc;
   }
-  if (ctx->resident) {
+  if (resident) {
     /* small lattices: whole iterations in shared memory, up to 1024 per launch */
     for (int64_t done = 0; done < n;) {
       const int m = (int)(n - done < 1024 ? n - done : 1024);
-      MICSA_CK(micsa_launch_resident(ctx->g, m, ctx->spin, ctx->dem0, ctx->dem1, ctx->jb,
+      MICSA_CK(micsa_launch_resident(ctx->g, ctx->resident, m, ctx->spin, ctx->dem0, ctx->dem1, ctx->jb,
                                      ctx->walk, ctx->stream));
       ctx->launches += 2;
       done += m;
@@ -1439,6 +1446,15 @@ int micsa_synchronize(micsa_ctx *ctx) {
     return fail(ctx, MICSA_ERR_CUDA,
                 "%u waits of the dataflow sweep timed out: the results of that iteration are "
                 "not valid", to);
+  }
+  if (ctx->resident > 1) {
+    MICSA_CK(micsa_cluster_timeout_count(&to));
+    if (to) {
+      MICSA_CK(micsa_cluster_timeout_clear());
+      return fail(ctx, MICSA_ERR_CUDA,
+                  "%u waits of the cluster-resident sweep timed out: the results of that "
+                  "iteration are not valid", to);
+    }
   }
   return MICSA_OK;
 }
@@ -1793,7 +1809,7 @@ int multi_setup(micsa_multi *m, micsa_ctx *const *ctxs, int n) {
     m->ctx.push_back(c);
     m->zc.push_back(multi_default_zc(c->g.L));
     m->pd.push_back(0);
-    /* a context whose samples fit one block's shared memory keeps its
+    /* a context whose samples fit the shared memory of a block or a cluster keeps its
      * resident kernel (whole iterations per launch, HBM touched only at the
      * ends) and runs it beside the mixed launch; MICSA_MULTI_RESIDENT=0 puts
      * it in the launch as well */
