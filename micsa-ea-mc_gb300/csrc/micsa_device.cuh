@@ -48,16 +48,17 @@ __device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
  * counts (j1 + 2*j2) + (j3 + 2*j4): accept iff 0 <= D + u - 3 <= 3, then
  * D <- D + u - 3 -- the function the reference's ISI boolean algebra
  * computes (main.cu:1037-1074), equal to it on all 64 inputs, in a
- * shorter circuit: T = D + u summed carry-save into bits s0 + 2 s1 + 4 s2
- * + 8 c3; accepted iff 3 <= T <= 6, i.e. !c3 and s2 ^ (s1 & s0); then
- * D0 = !s0 and D1 = s2 & (s0 | s1). */
+ * shorter circuit: T = D + u (0 ... 9) summed carry-save into bits s0 + 2 s1
+ * + 4 s2 (+ 8); accepted iff 3 <= T <= 6, i.e. s2 ^ (s1 & s0), which is 0
+ * for T = 8 and 9 as well (s2 = s1 = 0), so the eights are not formed; then
+ * D0 = !s0 and D1 = s0 ^ s1. */
 __device__ __forceinline__ uint32_t isi_update(uint32_t j1, uint32_t j2, uint32_t j3,
                                                uint32_t j4, uint32_t &D0, uint32_t &D1) {
   const uint32_t s0 = xor3(D0, j1, j3), c0 = maj3(D0, j1, j3);
   const uint32_t t = xor3(D1, j2, j4), cc = maj3(D1, j2, j4);
-  const uint32_t s1 = t ^ c0, s2 = lop3<0x78>(cc, t, c0), c3 = lop3<0x80>(cc, t, c0);
-  const uint32_t flip = lop3<0x78>(s2, s1, s0) & ~c3;
-  const uint32_t d1 = lop3<0xe0>(s2, s0, s1);
+  const uint32_t s1 = t ^ c0, s2 = lop3<0x78>(cc, t, c0);
+  const uint32_t flip = lop3<0x78>(s2, s1, s0);
+  const uint32_t d1 = s0 ^ s1;
   D0 = lop3<0x3a>(flip, s0, D0); /* flip ? !s0 : D0 */
   D1 = lop3<0xca>(flip, d1, D1); /* flip ? d1 : D1 */
   return flip;
