@@ -1647,6 +1647,20 @@ struct vcount {
     full(eights, e1, e2, f);
     ripple(f);
   }
+  /* eight words of weight 1 */
+  __device__ __forceinline__ void add_ones(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                           uint32_t a4, uint32_t a5, uint32_t a6, uint32_t a7) {
+    uint32_t c1, c2, c3, c4, d1, d2, e, f;
+    full(ones, a0, a1, c1);
+    full(ones, a2, a3, c2);
+    full(ones, a4, a5, c3);
+    full(ones, a6, a7, c4);
+    full(twos, c1, c2, d1);
+    full(twos, c3, c4, d2);
+    full(fours, d1, d2, e);
+    half(eights, e, f);
+    ripple(f);
+  }
   /* the bits of a count c = b0 + 2 b1 + 4 b2 (at most 7 per call) */
   __device__ __forceinline__ void add3(uint32_t b0, uint32_t b1, uint32_t b2) {
     uint32_t c1, c2, c3, c4;
@@ -1785,42 +1799,106 @@ k_demon_energy_cs(const micsa_geo g, const uint32_t *__restrict__ d0,
   for (int w = 0; w < W; w++) block_add(cnt[w].reduce(lane), buf, dem + (int64_t)s * g.nr + w * 32);
 }
 
-/* Overlap and C4 of the replica pairs (2k, 2k+1): with t = s(x) ^ s(x'),
- * bit 2k of t ^ (t >> 1) is d_x xor d_x', d = a xor b the pair difference.
- * blockIdx.y = axis*nd + dist (dist 0 also yields q via x' = x and the
- * second pass below), blockIdx.z = s*W + w.  Sites in natural order. */
-__global__ void __launch_bounds__(TPB)
-k_overlap(const micsa_geo g, const uint32_t *__restrict__ spin, unsigned long long *__restrict__ qd,
-          unsigned long long *__restrict__ c4d) {
-  const int nd = g.L / 2 + 1;
-  const int axis = blockIdx.y / nd, dist = blockIdx.y % nd;
-  const int s = blockIdx.z / g.W, w = blockIdx.z % g.W, lane = threadIdx.x & 31;
-  if (micsa_frozen(g, s)) return;
-  const int L = g.L, Lh = g.Lh, W = g.W;
-  const int64_t P = g.P, V = 2 * P;
-  const uint32_t *sp = spin + (int64_t)(s * 2) * P * W + w;
-  unsigned long long acc = 0, accq = 0;
-  const bool want_q = (axis == 0 && dist == 0);
-  const int64_t step = (int64_t)gridDim.x * TPB;
-  for (int64_t base = (int64_t)blockIdx.x * TPB + (threadIdx.x & ~31); base < V; base += step) {
-    const int64_t n = base + lane; /* V is a multiple of 32 */
-    const int x = (int)(n % L);
-    const int64_t q = n / L;
-    const int y = (int)(q % L), z = (int)(q / L);
-    int x2 = x, y2 = y, z2 = z;
-    if (axis == 0) { x2 += dist; if (x2 >= L) x2 -= L; }
-    else if (axis == 1) { y2 += dist; if (y2 >= L) y2 -= L; }
-    else { z2 += dist; if (z2 >= L) z2 -= L; }
-    const uint32_t s1 = __ldg(sp + ((int64_t)((x + y + z) & 1) * P + ((int64_t)z * L + y) * Lh + (x >> 1)) * W);
-    const uint32_t s2 = __ldg(sp + ((int64_t)((x2 + y2 + z2) & 1) * P + ((int64_t)z2 * L + y2) * Lh + (x2 >> 1)) * W);
-    const uint32_t t = s1 ^ s2;
-    acc += __popc(warp_transpose32(t ^ (t >> 1), lane));
-    if (want_q) accq += __popc(warp_transpose32(s1 ^ (s1 >> 1), lane));
+/* Overlap and C4 of the replica pairs (2k, 2k+1): with d the pair difference
+ * (bit of replica 2k xor that of 2k+1), the counts of d_x over all sites and
+ * of d_x ^ d_{x + r e_axis} for r = 1 .. L/2.
+ *
+ * The 16 pair bits of two replica words share one 32-bit word of d (even and
+ * odd bits).  A block takes 32 lines along an axis at a time -- one per lane,
+ * L words each, in shared memory with their first half repeated so that no
+ * index wraps -- for 32 distances: warp v has r0 = 32*chunk + 4v + 1 and the
+ * three after it, and counts eight positions of its line per step from the
+ * eight words there and eleven words r0 ahead, into one bit-sliced counter
+ * per distance; the counters become counts per pair once, after all the
+ * block's tiles (at most OV_CAP words per lane: the counters' capacity).
+ *
+ * Bound by the integer ALU pipe (about 4.5 logic operations per word, pair of
+ * words and distance).  A warp per 32 sites and one bit transpose per
+ * word and distance, the form before, with two 64-bit divisions per site,
+ * took 780 us at L=64, 2 samples x 64 replicas, where this takes 38. */
+constexpr int OV_CAP = 1023, OV_PITCH = 33, OV_R = 4, OV_CHUNK = OV_R * (TPB / 32);
+
+__device__ __forceinline__ uint32_t pair_bits(const uint32_t *sp, size_t site, int W, int w) {
+  const uint32_t *a = sp + site * W + w;
+  uint32_t s0, s1 = 0;
+  if (!(W & 1)) { /* w and the words per site are even: 8-byte aligned */
+    const uint2 v = __ldg((const uint2 *)a);
+    s0 = v.x;
+    s1 = v.y;
+  } else {
+    s0 = __ldg(a);
+    if (w + 1 < W) s1 = __ldg(a + 1);
   }
-  if (!(lane & 1)) {
-    const int k = w * 16 + (lane >> 1);
-    atomicAdd(c4d + (((int64_t)s * (g.nr / 2) + k) * 3 + axis) * nd + dist, acc);
-    if (want_q) atomicAdd(qd + (int64_t)s * (g.nr / 2) + k, accq);
+  return ((s0 ^ (s0 >> 1)) & 0x55555555u) | (((s1 ^ (s1 >> 1)) & 0x55555555u) << 1);
+}
+
+__global__ void __launch_bounds__(TPB, 2)
+k_overlap(const micsa_geo g, const int tiles, const uint32_t *__restrict__ spin,
+          unsigned long long *__restrict__ qd, unsigned long long *__restrict__ c4d) {
+  extern __shared__ uint32_t line[]; /* [L + L/2][OV_PITCH] */
+  const int L = g.L, Lh = g.Lh, W = g.W, nd = Lh + 1, PW = (W + 1) / 2;
+  const int axis = blockIdx.y % 3, chunk = blockIdx.y / 3;
+  const int s = blockIdx.z / PW, w0 = 2 * (blockIdx.z % PW);
+  if (micsa_frozen(g, s)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t P = (size_t)g.P;
+  const uint32_t *sp = spin + (size_t)(s * 2) * P * W;
+  const int r0 = OV_CHUNK * chunk + OV_R * warp + 1;
+  const bool want_q = axis == 0 && chunk == 0;
+  vcount cnt[OV_R], cq;
+  const int ntile = L * L / 32, t1 = min((int)(blockIdx.x + 1) * tiles, ntile);
+  for (int t = (int)blockIdx.x * tiles; t < t1; t++) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < 32 * L; i += TPB) {
+      /* consecutive threads along x, the direction contiguous in memory */
+      int pos, ln;
+      if (axis == 0) { ln = i / L; pos = i - ln * L; }
+      else { pos = i >> 5; ln = i & 31; }
+      const int id = 32 * t + ln, hi = id / L, lo = id - hi * L;
+      const int x = axis == 0 ? pos : lo, y = axis == 0 ? lo : (axis == 1 ? pos : hi),
+                z = axis == 2 ? pos : hi;
+      const size_t site = (size_t)((x + y + z) & 1) * P + (size_t)(z * L + y) * Lh + (x >> 1);
+      const uint32_t d = pair_bits(sp, site, W, w0);
+      line[pos * OV_PITCH + ln] = d;
+      if (pos < Lh) line[(pos + L) * OV_PITCH + ln] = d;
+    }
+    __syncthreads();
+    if (r0 <= Lh) {
+      /* r0 + 3 may pass L/2 in the last warp: those words lie in the line's
+       * repeated half up to L + L/2 - 1, and beyond it the counts are not used */
+      const int top = L + Lh - 1;
+#pragma unroll 1
+      for (int y0 = 0; y0 < L; y0 += 8) {
+        uint32_t a[8], b[8 + OV_R - 1];
+#pragma unroll
+        for (int k = 0; k < 8; k++) a[k] = line[(y0 + k) * OV_PITCH + lane];
+#pragma unroll
+        for (int k = 0; k < 8 + OV_R - 1; k++)
+          b[k] = line[min(y0 + r0 + k, top) * OV_PITCH + lane];
+#pragma unroll
+        for (int j = 0; j < OV_R; j++)
+          cnt[j].add_ones(a[0] ^ b[j], a[1] ^ b[j + 1], a[2] ^ b[j + 2], a[3] ^ b[j + 3],
+                          a[4] ^ b[j + 4], a[5] ^ b[j + 5], a[6] ^ b[j + 6], a[7] ^ b[j + 7]);
+      }
+    }
+    if (want_q)
+      for (int y0 = 8 * warp; y0 < L; y0 += 8 * (TPB / 32)) {
+        const uint32_t *a = line + y0 * OV_PITCH + lane;
+        cq.add_ones(a[0], a[OV_PITCH], a[2 * OV_PITCH], a[3 * OV_PITCH], a[4 * OV_PITCH],
+                    a[5 * OV_PITCH], a[6 * OV_PITCH], a[7 * OV_PITCH]);
+      }
+  }
+  const int wd = w0 + (lane & 1); /* the word of pair bit `lane` */
+  const int pair = wd * 16 + (lane >> 1);
+#pragma unroll
+  for (int j = 0; j < OV_R; j++)
+    if (r0 + j <= Lh) {
+      const unsigned long long v = cnt[j].reduce(lane);
+      if (wd < W) atomicAdd(c4d + (((int64_t)s * (g.nr / 2) + pair) * 3 + axis) * nd + r0 + j, v);
+    }
+  if (want_q) {
+    const unsigned long long v = cq.reduce(lane);
+    if (wd < W) atomicAdd(qd + (int64_t)s * (g.nr / 2) + pair, v);
   }
 }
 
@@ -2182,9 +2260,20 @@ cudaError_t micsa_launch_demon_energy(const micsa_geo &g, const uint32_t *d0, co
 
 cudaError_t micsa_launch_overlap(const micsa_geo &g, const uint32_t *spin, unsigned long long *qd,
                                  unsigned long long *c4d, cudaStream_t st) {
-  const int nd = g.L / 2 + 1;
-  dim3 grid(measure_blocks(2 * g.P, (int64_t)3 * nd * g.W * g.ns), 3 * nd, g.ns * g.W);
-  k_overlap<<<grid, TPB, 0, st>>>(g, spin, qd, c4d);
+  const int chunks = (g.Lh + OV_CHUNK - 1) / OV_CHUNK, PW = (g.W + 1) / 2, ntile = g.L * g.L / 32;
+  /* tiles per block: as many as leave two blocks per SM (the counters'
+   * reduction costs as much as a tile or two), within their capacity */
+  int64_t tiles = (int64_t)ntile * 3 * chunks * g.ns * PW / (2 * 152);
+  if (tiles > OV_CAP / g.L) tiles = OV_CAP / g.L;
+  if (tiles < 1) tiles = 1;
+  const size_t smem = sizeof(uint32_t) * OV_PITCH * (size_t)(g.L + g.Lh);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k_overlap, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 grid((unsigned)((ntile + tiles - 1) / tiles), 3 * chunks, g.ns * PW);
+  k_overlap<<<grid, TPB, smem, st>>>(g, (int)tiles, spin, qd, c4d);
   return cudaGetLastError();
 }
 
