@@ -2321,13 +2321,57 @@ __device__ __forceinline__ void xoshiro_step(uint64_t &s0, uint64_t &s1, uint64_
   s3 = rotl64(s3, 45);
 }
 
+/* One word's 64 draws from the generators' states before it, compared in
+ * full: the path of a word with a draw whose high half alone does not decide
+ * (k_refresh).  ring holds the word's new Fibonacci values; the values
+ * before it follow from x_{n-55} = x_n - x_{n-24}, highest slot first.  Rolled
+ * loops on a local array: rare, and it must not cost the caller registers. */
+__device__ __noinline__ void draw_word_exact(uint64_t *ring, uint64_t s0, uint64_t s1, uint64_t s2,
+                                             uint64_t s3, uint64_t z, uint64_t t0, uint64_t t1,
+                                             uint64_t t2, uint64_t *out) {
+  for (int b = 63; b >= 3; b--) /* slot b: x_{b-64} from x_{b-9} and x_{b-33} */
+    ring[b] = ring[(b - 9) & 63] - ring[(b - 33) & 63];
+  uint64_t d0 = 0, d1 = 0;
+  for (int b = 0; b < 64; b++) {
+    const uint64_t xo_out = rotl64(s0 + s3, 23) + s0;
+    xoshiro_step(s0, s1, s2, s3);
+    const uint64_t xn = ring[(b - 24) & 63] + ring[(b - 55) & 63];
+    const uint64_t pr = xn ^ ring[(b - 61) & 63];
+    ring[b] = xn;
+    z = z * REFRESH_LCG_A + 1;
+    const uint64_t e = (z + pr) + xo_out;
+    const uint32_t a0 = e < t0, a1 = e < t1, a2 = e < t2;
+    d0 |= (uint64_t)(a0 ^ a1 ^ a2) << b;
+    d1 |= (uint64_t)((a0 & a1) | (a0 & a2) | (a1 & a2)) << b;
+  }
+  out[0] = d0;
+  out[1] = d1;
+}
+
+/* The draw's sum e = z + pr + xo is compared by its high half alone, from the
+ * high halves of its four terms: with c the carry out of the low halves (0 to
+ * 3), e.hi = h + c.  x = (h + 4) / 2 (31 bits) against A = (T + 1) / 2, T the
+ * threshold's high half, decides unless x - A is 0, 1 or 2 (h within
+ * [T - 3, T]) or x is 0 or 1 (h + c may wrap): then the word is drawn again in
+ * full (12 of 2^31 draws).  The sign of x - A is the comparison's bit, the
+ * xor and the majority of three of them the demon's bits, and one funnel
+ * shift each collects them; the least of the x - A and x tells afterwards
+ * whether the word is to be redrawn.
+ *
+ * Bound by the integer ALU pipe: 28 such instructions per draw (jumps
+ * included) against 35 with 64-bit sums and compares; L=160, 2 x 64 streams:
+ * 5.5 ms against 6.9 (565 G draws/s), L=48, 4 x 64: 0.43 against 0.59.  The
+ * three differences as multiply-adds, off the ALU pipe, change nothing (5.6
+ * ms: three warps per scheduler do not fill both pipes). */
 template <int MINB>
 __global__ void __launch_bounds__(64, MINB)
 k_refresh(const micsa_geo g, const int first, const int count, const int64_t nwords,
           const int wps, const int64_t nseg, const uint64_t *__restrict__ rec,
           const uint64_t *__restrict__ lcg, const uint64_t *__restrict__ xoq,
           const uint64_t *__restrict__ fib, const uint64_t t0, const uint64_t t1,
-          const uint64_t t2, uint32_t *__restrict__ dem0, uint32_t *__restrict__ dem1) {
+          const uint64_t t2, const uint32_t A0, const uint32_t A1, const uint32_t A2,
+          uint32_t *__restrict__ dem0, uint32_t *__restrict__ dem1) {
+  __shared__ uint64_t before[5][64]; /* the states before the word, for a redraw */
   const int lane = threadIdx.x & 31;
   const int64_t warp = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (warp >= (int64_t)count * g.W * nseg) return; /* whole warps only */
@@ -2386,19 +2430,49 @@ k_refresh(const micsa_geo g, const int first, const int count, const int64_t nwo
   int a2 = (int)(hrem % mh), bb = (int)((hrem / mh) % m), c = (int)(hrem / ((int64_t)mh * m));
   int64_t base = ((int64_t)sample * 2 * g.nc + pi) * g.P * g.W + w;
   for (int64_t i = i0; i < i1; i++) {
-    uint64_t d0 = 0, d1 = 0;
+    before[0][threadIdx.x] = s0;
+    before[1][threadIdx.x] = s1;
+    before[2][threadIdx.x] = s2;
+    before[3][threadIdx.x] = s3;
+    before[4][threadIdx.x] = z;
+    uint64_t d0, d1;
+    {
+      uint32_t q0[2], q1[2], least = ~0u;
 #pragma unroll
-    for (int b = 0; b < 64; b++) {
-      const uint64_t xo_out = rotl64(s0 + s3, 23) + s0;
-      xoshiro_step(s0, s1, s2, s3);
-      const uint64_t xn = ring[(b - 24) & 63] + ring[(b - 55) & 63];
-      const uint64_t pr = xn ^ ring[(b - 61) & 63];
-      ring[b] = xn;
-      z = z * REFRESH_LCG_A + 1;
-      const uint64_t e = (z + pr) + xo_out;
-      const uint32_t a0 = e < t0, a1 = e < t1, a2 = e < t2;
-      d0 |= (uint64_t)(a0 ^ a1 ^ a2) << b;
-      d1 |= (uint64_t)((a0 & a1) | (a0 & a2) | (a1 & a2)) << b;
+      for (int h = 0; h < 2; h++) {
+        uint32_t c0 = 0, c1 = 0;
+#pragma unroll
+        for (int bb = 0; bb < 32; bb++) {
+          const int b = 32 * h + bb;
+          const uint64_t v = s0 + s3;
+          const uint32_t xo = __funnelshift_l((uint32_t)v, (uint32_t)(v >> 32), 23) + (uint32_t)(s0 >> 32);
+          xoshiro_step(s0, s1, s2, s3);
+          const uint64_t xn = ring[(b - 24) & 63] + ring[(b - 55) & 63];
+          const uint32_t pr = (uint32_t)(xn >> 32) ^ (uint32_t)(ring[(b - 61) & 63] >> 32);
+          ring[b] = xn;
+          z = z * REFRESH_LCG_A + 1;
+          const uint32_t x = ((uint32_t)(z >> 32) + pr + xo + 4) >> 1;
+          const uint32_t y0 = x - A0, y1 = x - A1, y2 = x - A2;
+          least = __vimin3_u32(least, y0, y1);
+          least = __vimin3_u32(least, y2, x);
+          c0 = __funnelshift_l(xor3(y0, y1, y2), c0, 1);
+          c1 = __funnelshift_l(maj3(y0, y1, y2), c1, 1);
+        }
+        q0[h] = __brev(c0);
+        q1[h] = __brev(c1);
+      }
+      d0 = (uint64_t)q0[0] | ((uint64_t)q0[1] << 32);
+      d1 = (uint64_t)q1[0] | ((uint64_t)q1[1] << 32);
+      if (__any_sync(FULL, least <= 2)) {
+        uint64_t old[64], out[2];
+#pragma unroll
+        for (int t = 0; t < 64; t++) old[t] = ring[t];
+        draw_word_exact(old, before[0][threadIdx.x], before[1][threadIdx.x],
+                        before[2][threadIdx.x], before[3][threadIdx.x], before[4][threadIdx.x], t0,
+                        t1, t2, out);
+        d0 = out[0];
+        d1 = out[1];
+      }
     }
     const uint32_t lo0 = warp_transpose32((uint32_t)d0, lane);
     const uint32_t hi0 = warp_transpose32((uint32_t)(d0 >> 32), lane);
@@ -2430,13 +2504,15 @@ cudaError_t micsa_launch_refresh(const micsa_geo &g, int first, int count, int64
                                  uint32_t *dem0, uint32_t *dem1, cudaStream_t st) {
   const int64_t warps = (int64_t)count * g.W * nseg;
   const unsigned blocks = (unsigned)((warps + 1) / 2);
+  uint32_t A[3];
+  for (int k = 0; k < 3; k++) A[k] = (uint32_t)(((thr[k] >> 32) + 1) >> 1);
   /* registers for 6 blocks (12 warps) per SM: 168, with a small spill */
   if (g.occ == 1)
     k_refresh<1><<<blocks, 64, 0, st>>>(g, first, count, nwords, wps, nseg, rec, lcg, xoq, fib,
-                                        thr[0], thr[1], thr[2], dem0, dem1);
+                                        thr[0], thr[1], thr[2], A[0], A[1], A[2], dem0, dem1);
   else
     k_refresh<6><<<blocks, 64, 0, st>>>(g, first, count, nwords, wps, nseg, rec, lcg, xoq, fib,
-                                        thr[0], thr[1], thr[2], dem0, dem1);
+                                        thr[0], thr[1], thr[2], A[0], A[1], A[2], dem0, dem1);
   return cudaGetLastError();
 }
 
