@@ -26,6 +26,8 @@
  *   MICSA_SWEEP_TILE, MICSA_SWEEP_TMA, MICSA_SWEEP_ASYNC, MICSA_SWEEP_PIPE,
  *   MICSA_SWEEP_FLOW, MICSA_SWEEP_QUAD   pin the sweep's launch shape at
  *                        micsa_create (meanings at micsa_tuning_report)
+ *   MICSA_SWEEP_CHAINS=K/U  with a pinned shape: samples in K chains of launches
+ *                        side by side, U iterations per graph replay
  *   MICSA_TUNE_CACHE=0   time every context instead of reusing the process's
  *                        choice for its shape
  *   MICSA_RESIDENT=0     keep L <= 32 on the per-half-sweep kernels
@@ -214,7 +216,9 @@ int micsa_profile(micsa_ctx *ctx, int64_t n, double *sweep_ms, double *iteration
  * tile=<default | row: blocks span whole rows along x>[/2: half-height
  * dataflow tiles]
  * fit=<iterations per launch of the dataflow sweep: its wavefront runs on
- * from one iteration into the next; 1 for the other loads> |
+ * from one iteration into the next; 1 for the other loads>
+ * chains=<K: the samples' launches in K chains side by side>/<iterations per
+ * graph replay> |
  * <zc>/<pd>/<split>/<occ>/<load 0|1|2|3|4|5|6 (6: pflow)>/<tile 0|1>:<ms per half-sweep> ...",
  * with " cached" before the "|" when the choice and its table were taken
  * over from an earlier context of the same device, L, nr, samples and nc in

@@ -18,6 +18,7 @@
 #include <string>
 #include <thread>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "micsa.h"
@@ -25,6 +26,7 @@
 #include "micsa_kernels.cuh"
 
 #define MICSA_TUNE_MAX 400
+#define MICSA_CHAINS_MAX 4
 
 struct micsa_ctx {
   micsa_config cfg;
@@ -53,6 +55,10 @@ struct micsa_ctx {
   int64_t resident_min = 1; /* calls of fewer iterations run half-sweep by half-sweep */
   int split = 0;           /* k > 0: half-sweep launches per group of k samples, group-major
                               (a smaller L2 working set); 0: all samples per launch */
+  int chains = 1;          /* an iteration's launches in the graph: chains of samples side by side */
+  int unit = 1;            /* iterations per replay of the iteration graph (per-half-sweep launches) */
+  cudaStream_t chain_st[MICSA_CHAINS_MAX - 1] = {nullptr}; /* captured from, for the chains */
+  cudaEvent_t chain_ev[MICSA_CHAINS_MAX] = {nullptr};
   micsa_tma tma = {};      /* tensor maps of the demon arrays (staged sweep) */
   int64_t graph_launches = 0; /* kernels per replay of the iteration graph */
   int ntune = 0;           /* launch shapes timed at creation */
@@ -212,11 +218,11 @@ void parallel_for(int64_t n, int64_t grain, F f) {
  * (s = 0, n = ns), or of a group -- the launch then sees only the group's
  * spins, couplings and demon planes through offset pointers. */
 cudaError_t launch_half(micsa_ctx *ctx, const micsa_geo &g, int s, int n, int p, int ic,
-                        int64_t *launches) {
+                        int64_t *launches, cudaStream_t st) {
   if (launches) ++*launches;
   if (s == 0 && n == g.ns)
     return micsa_launch_sweep_micsa(g, p, ic, ctx->spin, ctx->dem0, ctx->dem1, ctx->jb, ctx->walk,
-                                    &ctx->tma, ctx->stream);
+                                    &ctx->tma, st);
   const size_t PW = (size_t)g.P * g.W;
   micsa_geo g1 = g;
   g1.ns = n;
@@ -226,7 +232,7 @@ cudaError_t launch_half(micsa_ctx *ctx, const micsa_geo &g, int s, int n, int p,
                                   ctx->dem0 + s * 2 * (size_t)g.nc * PW,
                                   ctx->dem1 + s * 2 * (size_t)g.nc * PW,
                                   ctx->jb + (size_t)s * 2 * g.P, ctx->walk + s, &ctx->tma,
-                                  ctx->stream);
+                                  st);
 }
 
 /* The half-sweeps of one iteration (ic = ic0 .. ic1-1).  split = 0: plane by
@@ -247,9 +253,60 @@ cudaError_t launch_halves(micsa_ctx *ctx, const micsa_geo &g, int split, int ic0
   for (int s = 0; s < g.ns; s += k)
     for (int ic = ic0; ic < ic1; ic++)
       for (int p = 0; p < 2; p++)
-        if ((e = launch_half(ctx, g, s, s + k <= g.ns ? k : g.ns - s, p, ic, launches)) !=
-            cudaSuccess)
+        if ((e = launch_half(ctx, g, s, s + k <= g.ns ? k : g.ns - s, p, ic, launches,
+                             ctx->stream)) != cudaSuccess)
           return e;
+  return e;
+}
+
+/* iters iterations of the per-half-sweep launches with the samples in K
+ * chains side by side, for a stream capture on the context's stream: chain c
+ * takes the samples ns*c/K .. ns*(c+1)/K - 1 through all half-sweeps (and,
+ * with walks, the walk's step after each iteration) on a stream of its own,
+ * so that while one chain's launch drains the other's fills the GPU.  Samples
+ * are independent: no chain waits for another until the end. */
+cudaError_t launch_chains(micsa_ctx *ctx, const micsa_geo &g, int K, int iters, bool walks,
+                          int64_t *launches) {
+  cudaError_t e = cudaSuccess;
+  for (int c = 0; c < K && e == cudaSuccess; c++)
+    if (!ctx->chain_ev[c]) e = cudaEventCreateWithFlags(&ctx->chain_ev[c], cudaEventDisableTiming);
+  cudaStream_t st[MICSA_CHAINS_MAX] = {ctx->stream};
+  if (e == cudaSuccess && K > 1) e = cudaEventRecord(ctx->chain_ev[0], ctx->stream);
+  for (int c = 1; c < K && e == cudaSuccess; c++) {
+    st[c] = ctx->chain_st[c - 1];
+    e = cudaStreamWaitEvent(st[c], ctx->chain_ev[0], 0);
+  }
+  for (int it = 0; it < iters; it++)
+    for (int h = 0; h <= 2 * g.nc; h++)
+      for (int c = 0; c < K && e == cudaSuccess; c++) {
+        const int s0 = g.ns * c / K, n = g.ns * (c + 1) / K - s0;
+        if (h < 2 * g.nc) {
+          e = launch_half(ctx, g, s0, n, h & 1, h >> 1, launches, st[c]);
+        } else if (walks) {
+          micsa_geo g1 = g;
+          g1.ns = n;
+          g1.active = g.active ? g.active + s0 : nullptr;
+          e = micsa_launch_walk_advance(g1, ctx->walk + s0, st[c]);
+          if (launches) ++*launches;
+        }
+      }
+  /* joined even after an error, so that the capture can end */
+  for (int c = 1; c < K; c++) {
+    if (!st[c]) continue;
+    cudaError_t j = cudaEventRecord(ctx->chain_ev[c], st[c]);
+    if (j == cudaSuccess) j = cudaStreamWaitEvent(ctx->stream, ctx->chain_ev[c], 0);
+    if (e == cudaSuccess) e = j;
+  }
+  return e;
+}
+
+/* streams for K chains (outside any capture) */
+cudaError_t ensure_chains(micsa_ctx *ctx, int K) {
+  int least = 0, greatest = 0;
+  cudaError_t e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+  for (int c = 0; c + 1 < K && e == cudaSuccess; c++)
+    if (!ctx->chain_st[c])
+      e = cudaStreamCreateWithPriority(&ctx->chain_st[c], cudaStreamNonBlocking, greatest);
   return e;
 }
 
@@ -258,7 +315,7 @@ cudaError_t launch_halves(micsa_ctx *ctx, const micsa_geo &g, int split, int ic0
  * choice and table instead of timing again, so batches and servers that open
  * many contexts of a few shapes pay for each shape once. */
 struct tune_entry {
-  int zc, pd, split, occ, tma, async, pipe, tw, flow, quad, fit, pers, half, xs, n;
+  int zc, pd, split, occ, tma, async, pipe, tw, flow, quad, fit, pers, half, xs, chains, unit, n;
   std::vector<int> zcs, pds, splits, occs, loads, tws;
   std::vector<double> ms;
 };
@@ -316,6 +373,14 @@ int autotune(micsa_ctx *ctx) {
       const int k = atoi(ek);
       if (g.flow && k >= 1 && k <= 64) g.fit = k;
     }
+    if (const char *eh = getenv("MICSA_SWEEP_CHAINS")) {
+      /* K or K/U: chains, iterations per graph replay */
+      int K = atoi(eh), U = strchr(eh, '/') ? atoi(strchr(eh, '/') + 1) : 1;
+      K = K < 1 ? 1 : (K > MICSA_CHAINS_MAX ? MICSA_CHAINS_MAX : K);
+      ctx->chains = g.flow || ctx->split ? 1 : (K < g.ns ? K : g.ns);
+      ctx->unit = g.flow || U < 1 ? 1 : (U > 64 ? 64 : U);
+      MICSA_CK(ensure_chains(ctx, ctx->chains));
+    }
     const int oc = eo ? atoi(eo) : 3;
     g.occ = g.pipe ? (oc == 2 ? 2 : 3) : (oc == 4 ? 4 : 3);
     ctx->ntune = 0;
@@ -342,6 +407,9 @@ int autotune(micsa_ctx *ctx) {
       g.pers = t.pers;
       g.half = t.half;
       g.xs = t.xs;
+      ctx->chains = t.chains;
+      ctx->unit = t.unit;
+      MICSA_CK(ensure_chains(ctx, ctx->chains));
       ctx->ntune = t.n;
       for (int c = 0; c < t.n; c++) {
         ctx->tune_zc[c] = t.zcs[c];
@@ -540,6 +608,7 @@ int autotune(micsa_ctx *ctx) {
   g.pers = best_pers;
   g.quad = best_quad;
   g.fit = 1;
+  double best_flow_it = 1e30;
   if (g.flow) {
     /* iterations per dataflow launch: the wavefront runs on from one
      * iteration into the next instead of draining the GPU at every launch
@@ -600,8 +669,92 @@ int autotune(micsa_ctx *ctx) {
       if (te == cudaSuccess) te = cudaEventElapsedTime(&ms, e0, e1);
       cudaGraphExecDestroy(ge);
       MICSA_CK(te);
-      if (ms / ((double)rr * g.fit) >= best_it) g.half = 0;
+      const double hit = ms / ((double)rr * g.fit);
+      if (hit >= best_it) g.half = 0;
+      else best_it = hit;
     }
+    best_flow_it = best_it;
+  }
+  /* Samples in chains side by side, and several iterations per graph replay,
+   * with the two fastest shapes that launch all samples at once.  One chain
+   * leaves the GPU to drain after every half-sweep; two hide it (L=96, 8
+   * samples x 32 replicas: 218 -> 174 us per iteration; L=48, 32 x 64: 193 ->
+   * 158; L=128, 2 x 64: 160 against 176 for the dataflow sweep), four and
+   * several iterations per replay help the smallest launches (L=48, 4 x 64:
+   * 43.6 -> 38.9 with two chains and four iterations). */
+  {
+    double base = 1e30; /* ms per iteration of the choice so far */
+    if (g.flow) base = best_flow_it;
+    int two[2], nt = 0;
+    for (int c = 0; c < n && c < MICSA_TUNE_MAX; c++) {
+      if (ctx->tune_load[c] == 4 || ctx->tune_load[c] == 6 || ctx->tune_split[c]) continue;
+      if (nt < 2) two[nt++] = c;
+      else if (ctx->tune_ms[c] < ctx->tune_ms[two[1]]) two[1] = c;
+      if (nt == 2 && ctx->tune_ms[two[1]] < ctx->tune_ms[two[0]]) std::swap(two[0], two[1]);
+    }
+    const micsa_geo chosen = g;
+    micsa_geo pick = g;
+    int pick_split = ctx->split, pick_chains = 1, pick_unit = 1;
+    auto time_chains = [&](int K, int U, double *per) -> int {
+      cudaGraph_t gr = nullptr;
+      cudaGraphExec_t ge = nullptr;
+      MICSA_CK(ensure_chains(ctx, K));
+      MICSA_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+      const cudaError_t le = launch_chains(ctx, g, K, U, true, nullptr);
+      const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &gr);
+      MICSA_CK(le);
+      MICSA_CK(ce);
+      const cudaError_t ie = cudaGraphInstantiate(&ge, gr, 0);
+      cudaGraphDestroy(gr);
+      MICSA_CK(ie);
+      const int nrep = 24 / U;
+      float ms = 0;
+      cudaError_t te = cudaGraphLaunch(ge, ctx->stream);
+      if (te == cudaSuccess) te = cudaEventRecord(e0, ctx->stream);
+      for (int rep = 0; rep < nrep && te == cudaSuccess; rep++) te = cudaGraphLaunch(ge, ctx->stream);
+      if (te == cudaSuccess) te = cudaEventRecord(e1, ctx->stream);
+      if (te == cudaSuccess) te = cudaEventSynchronize(e1);
+      if (te == cudaSuccess) te = cudaEventElapsedTime(&ms, e0, e1);
+      cudaGraphExecDestroy(ge);
+      MICSA_CK(te);
+      *per = ms / (double)(nrep * U);
+      return MICSA_OK;
+    };
+    if (!g.flow && ctx->split) { /* sample-major launches: their own time */
+      double per = 0;
+      if ((rc = time_shape(ctx->split, 3 * reps, &per))) return rc;
+      base = per * 2 * g.nc;
+    }
+    for (int k = 0; k < nt; k++)
+      for (int K : {1, 2, 4})
+        for (int U : {1, 4}) {
+          if (K > g.ns) continue;
+          const int c = two[k], tm = ctx->tune_load[c];
+          g = chosen;
+          g.flow = g.pers = g.half = g.xs = 0;
+          g.fit = 1;
+          g.zc = ctx->tune_zc[c];
+          g.pd = ctx->tune_pd[c];
+          g.occ = ctx->tune_occ[c];
+          g.tma = tm == 1;
+          g.async = tm == 2;
+          g.pipe = tm == 3;
+          g.quad = tm == 5;
+          g.tw = ctx->tune_tw[c];
+          double per = 0;
+          if ((rc = time_chains(K, U, &per))) return rc;
+          if (per < base) {
+            base = per;
+            pick = g;
+            pick_split = 0;
+            pick_chains = K;
+            pick_unit = U;
+          }
+        }
+    g = pick;
+    ctx->split = pick_split;
+    ctx->chains = pick_chains;
+    ctx->unit = pick_unit;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -621,6 +774,8 @@ int autotune(micsa_ctx *ctx) {
     t.pers = g.pers;
     t.half = g.half;
     t.xs = g.xs;
+    t.chains = ctx->chains;
+    t.unit = ctx->unit;
     t.n = n;
     t.zcs.assign(ctx->tune_zc, ctx->tune_zc + n);
     t.pds.assign(ctx->tune_pd, ctx->tune_pd + n);
@@ -655,11 +810,16 @@ int enqueue_micsa_iteration(micsa_ctx *ctx, int64_t *launches) {
 }
 
 /* the iteration graph of k iterations */
+int enqueue_for_graph(micsa_ctx *ctx, int k, int64_t *launches) {
+  if (ctx->g.flow || ctx->split) return enqueue_micsa_iterations(ctx, k, launches);
+  MICSA_CK(launch_chains(ctx, ctx->g, ctx->chains, k, true, launches));
+  return MICSA_OK;
+}
 int capture_iterations(micsa_ctx *ctx, int k, cudaGraph_t *graph, cudaGraphExec_t *exec,
                        int64_t *launches) {
   MICSA_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   *launches = 0;
-  int rc = enqueue_micsa_iterations(ctx, k, launches);
+  int rc = enqueue_for_graph(ctx, k, launches);
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
   if (rc) {
@@ -809,12 +969,13 @@ int micsa_create(const micsa_config *cfg, micsa_ctx **out) {
 
 int micsa_tuning_report(const micsa_ctx *ctx, char *buf, size_t n) {
   if (!ctx || !buf || n == 0) return MICSA_ERR_ARG;
-  int k = snprintf(buf, n, "zc=%d pd=%d split=%d occ=%d load=%s tile=%s%s%s fit=%d%s |", ctx->g.zc,
+  int k = snprintf(buf, n, "zc=%d pd=%d split=%d occ=%d load=%s tile=%s%s%s fit=%d chains=%d/%d%s |", ctx->g.zc,
                    ctx->g.pd, ctx->split, ctx->g.occ,
                    ctx->g.tma ? "tma" : (ctx->g.async ? "async" : (ctx->g.pipe ? "pipe" : (ctx->g.flow ? (ctx->g.pers ? "pflow" : "flow") : (ctx->g.quad ? "quad" : "direct")))),
                    ctx->g.tw ? "row" : "default", ctx->g.flow && ctx->g.half ? "/2" : "",
                    ctx->g.flow && ctx->g.xs ? "+xs" : "",
-                   ctx->g.flow ? ctx->g.fit : 1,
+                   ctx->g.flow ? ctx->g.fit : 1, ctx->g.flow || ctx->split ? 1 : ctx->chains,
+                   ctx->g.flow ? ctx->g.fit : ctx->unit,
                    ctx->tune_cached ? " cached" : "");
   for (int c = 0; c < ctx->ntune && k > 0 && (size_t)k < n; c++)
     k += snprintf(buf + k, n - (size_t)k, " %d/%d/%d/%d/%d/%d:%.5fms", ctx->tune_zc[c],
@@ -850,6 +1011,10 @@ int micsa_destroy(micsa_ctx *ctx) {
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
+  for (cudaStream_t st : ctx->chain_st)
+    if (st) cudaStreamDestroy(st);
+  for (cudaEvent_t e : ctx->chain_ev)
+    if (e) cudaEventDestroy(e);
   micsa_refresh_plan_free(&ctx->plan);
   if (ctx->rec_host) cudaFreeHost(ctx->rec_host);
   if (ctx->rec_copied) cudaEventDestroy(ctx->rec_copied);
@@ -1242,9 +1407,9 @@ int micsa_iterate(micsa_ctx *ctx, int64_t n) {
   /* the graph replays ctx->g.fit iterations at a time (the dataflow sweep may
    * carry several per launch); the remainder k < fit runs as one launch of k
    * iterations, from a graph made on first use */
-  const int unit = ctx->g.flow && ctx->g.fit > 1 ? ctx->g.fit : 1;
+  const int unit = ctx->g.flow ? (ctx->g.fit > 1 ? ctx->g.fit : 1) : ctx->unit;
   const bool resident = ctx->resident && (n >= ctx->resident_min || n == 0);
-  if (!ctx->graph_exec && !resident &&
+  if (!ctx->graph_exec && !resident && n >= unit &&
       (rc = capture_iterations(ctx, unit, &ctx->graph, &ctx->graph_exec, &ctx->graph_launches)))
     return rc;
   const int left = unit > 1 ? (int)(n % unit) : 0;
@@ -1383,7 +1548,9 @@ int micsa_profile(micsa_ctx *ctx, int64_t n, double *sweep_ms, double *iteration
   cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     e = cudaEventRecordWithFlags(ev[0], ctx->stream, cudaEventRecordExternal);
-    if (e == cudaSuccess) e = launch_halves(ctx, g, ctx->split, 0, g.nc, &nl);
+    if (e == cudaSuccess)
+      e = g.flow || ctx->split ? launch_halves(ctx, g, ctx->split, 0, g.nc, &nl)
+                               : launch_chains(ctx, g, ctx->chains, 1, false, &nl);
     if (e == cudaSuccess) e = cudaEventRecordWithFlags(ev[1], ctx->stream, cudaEventRecordExternal);
     if (e == cudaSuccess)
       e = unit > 1 ? micsa_launch_walk_add(g, ctx->walk, unit, ctx->stream)
