@@ -840,7 +840,7 @@ int64_t micsa_footprint_bytes(const micsa_config *cfg) {
   char msg[128];
   if (check_cfg(cfg, msg, sizeof msg) != MICSA_OK) return -1;
   sizes s = sizes_of(*cfg);
-  return 4 * (s.spin_w + 2 * s.dem_w + s.rnd_w) + s.jb_b + 8 * (s.stage_w + s.acc_w) + 4096 +
+  return 4 * (s.spin_w + 2 * s.dem_w + s.rnd_w) + s.jb_b + 8 * (s.stage_w + s.acc_w) + MICSA_LUT_BYTES +
          4 * (9 * (int64_t)cfg->nr) + 4 * MICSA_MAX_SAMPLES;
 }
 
@@ -922,7 +922,7 @@ int micsa_create(const micsa_config *cfg, micsa_ctx **out) {
   MICSA_CK_CREATE(cudaMalloc(&ctx->dem1, 4 * s.dem_w));
   MICSA_CK_CREATE(cudaMalloc(&ctx->rnd, 4 * s.rnd_w));
   MICSA_CK_CREATE(cudaMalloc(&ctx->jb, s.jb_b));
-  MICSA_CK_CREATE(cudaMalloc(&ctx->lut, 4096));
+  MICSA_CK_CREATE(cudaMalloc(&ctx->lut, MICSA_LUT_BYTES));
   MICSA_CK_CREATE(cudaMalloc(&ctx->te, 4 * 8 * (size_t)cfg->nr));
   MICSA_CK_CREATE(cudaMalloc(&ctx->keys, 4 * (size_t)cfg->nr));
   MICSA_CK_CREATE(cudaMalloc(&ctx->walk, sizeof(int) * MICSA_MAX_SAMPLES));
@@ -1044,7 +1044,10 @@ int micsa_set_lut(micsa_ctx *ctx, const void *lut, size_t bytes) {
       return fail(ctx, MICSA_ERR_ARG, "LUT prebisection entry %d has min > max", i);
   int rc = set_device(ctx);
   if (rc) return rc;
-  MICSA_CK(cudaMemcpyAsync(ctx->lut, lut, 4096, cudaMemcpyHostToDevice, ctx->stream));
+  std::vector<uint32_t> both(MICSA_LUT_BYTES / 4);
+  memcpy(both.data(), lut, 4096);
+  micsa_lut_bins(lut, both.data() + 1024);
+  MICSA_CK(cudaMemcpyAsync(ctx->lut, both.data(), MICSA_LUT_BYTES, cudaMemcpyHostToDevice, ctx->stream));
   MICSA_CK(cudaStreamSynchronize(ctx->stream));
   ctx->have_lut = 1;
   return MICSA_OK;
@@ -1389,11 +1392,17 @@ int micsa_monte_carlo(micsa_ctx *ctx, int flag, const uint32_t *te, const uint32
   if (!te || !keys) return fail(ctx, MICSA_ERR_ARG, "flag 0 needs counters and keys");
   if (!ctx->have_lut) return fail(ctx, MICSA_ERR_STATE, "no LUT uploaded");
   if ((rc = ready_for_sweeps(ctx, 0))) return rc;
-  MICSA_CK(cudaMemcpyAsync(ctx->te, te, 4 * 8 * (size_t)g.nr, cudaMemcpyHostToDevice, ctx->stream));
-  MICSA_CK(cudaMemcpyAsync(ctx->keys, keys, 4 * (size_t)g.nr, cudaMemcpyHostToDevice, ctx->stream));
+  const bool values = g.nr <= MICSA_RND_VALUES;
+  if (!values) {
+    MICSA_CK(cudaMemcpyAsync(ctx->te, te, 4 * 8 * (size_t)g.nr, cudaMemcpyHostToDevice, ctx->stream));
+    MICSA_CK(cudaMemcpyAsync(ctx->keys, keys, 4 * (size_t)g.nr, cudaMemcpyHostToDevice, ctx->stream));
+  }
   for (int p = 0; p < 2; p++) {
-    MICSA_CK(micsa_launch_gen_rnd(g, p, ctx->te + 4 * g.nr * p, ctx->keys, ctx->lut, ctx->rnd,
-                                  ctx->stream));
+    if (values)
+      MICSA_CK(micsa_launch_gen_rnd_values(g, p, te + 4 * g.nr * p, keys, ctx->lut, ctx->rnd, ctx->stream));
+    else
+      MICSA_CK(micsa_launch_gen_rnd(g, p, ctx->te + 4 * g.nr * p, ctx->keys, ctx->lut, ctx->rnd,
+                                    ctx->stream));
     MICSA_CK(micsa_launch_sweep_metropolis(g, p, ctx->spin, ctx->jb, ctx->rnd, ctx->stream));
   }
   ctx->launches += 4;

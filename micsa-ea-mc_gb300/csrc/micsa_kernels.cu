@@ -108,18 +108,17 @@ __device__ __forceinline__ void prefetch_l2(const uint32_t *a) {
 /* ------------------------------------------------------------ geometry */
 struct site_xyz { int x, y, z; };
 
-/* real site of the reference word (colour p, h, bit b) (ini.c:317-337) */
-__device__ __forceinline__ site_xyz ref_site(const micsa_geo &g, int p, int64_t h, int b) {
-  const int m = g.L >> 2, mh = m >> 1;
-  const int a2 = (int)(h % mh);
-  const int64_t q = h / mh;
-  const int bb = (int)(q % m);
-  const int c = (int)(q / m);
-  const int a = 2 * a2 + ((bb + c + p) & 1);
+/* real site of the reference word (colour p, h, bit b) (ini.c:317-337); the
+ * site of bit b + 32 is L/2 planes above */
+__device__ __forceinline__ site_xyz ref_site(const micsa_geo &g, int p, uint32_t h, int b) {
+  const uint32_t m = (uint32_t)g.L >> 2, mh = m >> 1;
+  const uint32_t q = h / mh, a2 = h - q * mh;
+  const uint32_t c = q / m, bb = q - c * m;
+  const uint32_t a = 2 * a2 + ((bb + c + (uint32_t)p) & 1);
   site_xyz s;
-  s.x = (b & 3) * m + a;
-  s.y = ((b >> 2) & 3) * m + bb;
-  s.z = (b >> 4) * m + c;
+  s.x = (b & 3) * (int)m + (int)a;
+  s.y = ((b >> 2) & 3) * (int)m + (int)bb;
+  s.z = (b >> 4) * (int)m + (int)c;
   return s;
 }
 
@@ -1456,66 +1455,144 @@ __device__ __forceinline__ uint32_t lut_bisect(uint32_t hi, uint32_t lo, const u
 #undef MICSA_BELOW
 }
 
-/* one 32-bit word of Bernoulli bits from one Philox call, with the
- * reference's counter bump, post-mix and rotation (main.cu:597-644) */
-__device__ __forceinline__ uint32_t heat_bath_word(uint32_t (&c)[4], uint32_t k0, uint32_t k1,
-                                                   const uint32_t *thr, const uint16_t *pre) {
-  uint32_t v[4] = {c[0], c[1], c[2], c[3]};
+/* one Philox call with the reference's counter bump and post-mix
+ * (main.cu:597-644): four 64-bit uniforms (v[k] high, l[k] low) and the
+ * rotation of the word their bytes make */
+__device__ __forceinline__ uint32_t heat_bath_uniforms(uint32_t (&c)[4], uint32_t k0, uint32_t k1,
+                                                       uint32_t (&v)[4], uint32_t (&l)[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) v[k] = c[k];
   philox10(v, k0, k1);
   c[0]++;
   const uint32_t hi = v[0] ^ v[2], lo = v[1] ^ v[3];
-  uint32_t l[4];
   l[0] = ((v[1] << 17) | (v[0] >> 15)) ^ hi ^ ((hi << 21) | (lo >> 11));
   l[1] = ((v[0] << 17) | (v[1] >> 15)) ^ lo ^ (lo << 21);
   l[2] = (hi << 28) | (lo >> 4);
   l[3] = (lo << 28) | (hi >> 4);
-  const uint32_t rot = (l[0] + v[1] + l[2] + v[3]) >> 27;
-  uint32_t bb = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) bb |= lut_bisect(v[k], l[k], thr, pre) << (8 * k);
-  return __funnelshift_l(bb, bb, rot);
+  return (l[0] + v[1] + l[2] + v[3]) >> 27;
 }
 
 /* Thread (h, r) = tid = h*nr + r, exactly the reference's thread id, key
- * (tid, keys[r]) and counter te[r] with z += tid; the three 64-bit words
- * (bit = block) are transposed in-warp to replica words of the 64 sites. */
-__global__ void __launch_bounds__(TPB)
-k_gen_rnd(const micsa_geo g, const int p, const uint32_t *__restrict__ te,
-          const uint32_t *__restrict__ keys, const uint8_t *__restrict__ lut,
-          uint32_t *__restrict__ rnd) {
-  __shared__ uint32_t s_thr[512];
-  __shared__ uint16_t s_pre[1024];
-  const uint32_t *lw = reinterpret_cast<const uint32_t *>(lut);
-  for (int t = threadIdx.x; t < 1024; t += TPB) {
-    const uint32_t v = lw[t];
-    if (t < 512) s_thr[t] = v;
-    else {
-      s_pre[2 * (t - 512)] = (uint16_t)(v & 0xffffu);
-      s_pre[2 * (t - 512) + 1] = (uint16_t)(v >> 16);
-    }
+ * (tid, keys[r]) and counter te[r] with z += tid, draws three 64-bit words (two
+ * Philox calls and 8 bytes each; bit = block), which are
+ * transposed in-warp to replica words of the 64 sites.
+ *
+ * Each byte is the index of the first threshold above a 64-bit uniform.  Of
+ * the 1024 bins of its top 10 bits most hold at most one threshold: there one
+ * comparison of the high halves decides between the two indices of the bin's
+ * entry (micsa_lut_bins).  The others -- bins with several thresholds, the
+ * bin of threshold 254 above which the index is 255, equal high halves -- are
+ * collected per warp and bisected 32 at a time: 2% of the draws with the
+ * heat-bath LUT, which bisected in place kept whole warps in the loop for
+ * nearly every byte.
+ *
+ * Bound by latency at the sizes that thermalise (six warps per scheduler at
+ * L=64, 64 replicas, 45% of the issue slots): 13.7 us per colour there, 15.9
+ * with the bisection in place and 64-bit site divisions, 14.2 with a thread
+ * per 64-bit word (the prologue three times). */
+constexpr int RND_QUEUE = 32 + 128; /* waiting draws per warp: fewer than 32, plus one call's */
+
+/* counters and keys: device arrays, or with the launch's arguments (staged in
+ * shared memory by the block: lanes reading argument memory at addresses of
+ * their own are served one after another) */
+struct rnd_arrays {
+  static constexpr int STAGE = 1;
+  const uint32_t *te, *keys;
+  __device__ __forceinline__ void stage(uint4 *, uint32_t *, int) const {}
+  __device__ __forceinline__ uint4 counter(int r, const uint4 *) const { return ((const uint4 *)te)[r]; }
+  __device__ __forceinline__ uint32_t key(int r, const uint32_t *) const { return keys[r]; }
+};
+struct rnd_values {
+  static constexpr int STAGE = MICSA_RND_VALUES;
+  uint4 te[MICSA_RND_VALUES];
+  uint32_t keys[MICSA_RND_VALUES];
+  __device__ __forceinline__ void stage(uint4 *t, uint32_t *k, int nr) const {
+    if ((int)threadIdx.x < nr) t[threadIdx.x] = te[threadIdx.x];
+    if ((int)threadIdx.x < nr) k[threadIdx.x] = keys[threadIdx.x];
   }
+  __device__ __forceinline__ uint4 counter(int r, const uint4 *t) const { return t[r]; }
+  __device__ __forceinline__ uint32_t key(int r, const uint32_t *k) const { return k[r]; }
+};
+static_assert(MICSA_RND_VALUES <= TPB, "one thread stages one replica");
+
+template <class Source>
+__global__ void __launch_bounds__(TPB)
+k_gen_rnd(const __grid_constant__ micsa_geo g, const int p, const __grid_constant__ Source from,
+          const uint8_t *__restrict__ lut, uint32_t *__restrict__ rnd) {
+  __shared__ uint4 s_bin4[512]; /* threshold's high half; index below | index above << 8 | open << 16 */
+  __shared__ uint2 s_q[TPB / 32][RND_QUEUE];
+  __shared__ uint8_t s_qid[TPB / 32][RND_QUEUE];
+  __shared__ uint4 s_te[Source::STAGE];
+  __shared__ uint32_t s_key[Source::STAGE];
+  __shared__ uint8_t s_late[TPB / 32][2 * 32 * 4]; /* bytes found by bisection, [call][lane][byte] */
+  const uint4 *bins = reinterpret_cast<const uint4 *>(lut + 4096);
+  for (int t = threadIdx.x; t < 512; t += TPB) s_bin4[t] = __ldg(bins + t);
+  const uint2 *s_bin = reinterpret_cast<const uint2 *>(s_bin4);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t *late = (uint32_t *)s_late[warp];
+  late[lane] = late[32 + lane] = 0;
+  /* H*nr = P*W/2 < 2^31 (checked at creation) */
+  const uint32_t tid = blockIdx.x * TPB + threadIdx.x, h = tid / (uint32_t)g.nr;
+  const int r = (int)(tid - h * (uint32_t)g.nr);
+  from.stage(s_te, s_key, g.nr);
   __syncthreads();
-  const int64_t tid = (int64_t)blockIdx.x * TPB + threadIdx.x;
-  if (tid >= g.H * g.nr) return; /* warp-uniform: H*nr is a multiple of 32 */
-  const int lane = threadIdx.x & 31;
-  const int r = (int)(tid % g.nr);
-  const int64_t h = tid / g.nr;
-  uint32_t c[4] = {te[4 * r], te[4 * r + 1], te[4 * r + 2] + (uint32_t)tid, te[4 * r + 3]};
-  const uint32_t key1 = keys[r];
-  uint32_t wd[6];
+  if (tid >= (uint32_t)g.H * (uint32_t)g.nr) return; /* warp-uniform: H*nr is a multiple of 32 */
+  const uint4 t4 = from.counter(r, s_te);
+  uint32_t c[4] = {t4.x, t4.y, t4.z + tid, t4.w};
+  const uint32_t key1 = from.key(r, s_key);
+  const site_xyz site = ref_site(g, p, h, lane);
+  uint32_t *out = rnd + (((int64_t)site.z * g.L + site.y) * g.Lh + (site.x >> 1)) * g.W + (r >> 5);
+  int waiting = 0; /* draws in the warp's queue */
+  auto bisect32 = [&](int at) { /* queue entries at .. at+31, as far as there are any */
+    __syncwarp();
+    if (at + lane < waiting) {
+      const uint2 u = s_q[warp][at + lane];
+      s_late[warp][s_qid[warp][at + lane]] =
+          (uint8_t)lut_bisect(u.x, u.y, reinterpret_cast<const uint32_t *>(lut),
+                              reinterpret_cast<const uint16_t *>(lut + 2048));
+    }
+    __syncwarp();
+  };
+#pragma unroll 1
+  for (int word = 0; word < 3; word++) {
+    uint32_t rot[2], wd[2];
 #pragma unroll
-  for (int q = 0; q < 6; q++) wd[q] = heat_bath_word(c, (uint32_t)tid, key1, s_thr, s_pre);
-  const site_xyz a = ref_site(g, p, h, lane), b = ref_site(g, p, h, lane + 32);
-  const int64_t ia = ((int64_t)a.z * g.L + a.y) * g.Lh + (a.x >> 1);
-  const int64_t ib = ((int64_t)b.z * g.L + b.y) * g.Lh + (b.x >> 1);
-  const int w = r >> 5;
+    for (int q = 0; q < 2; q++) {
+      uint32_t v[4], l[4], bb = 0;
+      rot[q] = heat_bath_uniforms(c, tid, key1, v, l);
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    /* 64-bit word k = (wd[2k] << 32) | wd[2k+1]; bit b = block b */
-    const uint32_t lo = warp_transpose32(wd[2 * k + 1], lane);
-    const uint32_t hi = warp_transpose32(wd[2 * k], lane);
-    rnd[((int64_t)k * g.P + ia) * g.W + w] = lo;
-    rnd[((int64_t)k * g.P + ib) * g.W + w] = hi;
+      for (int k = 0; k < 4; k++) {
+        const uint2 e = s_bin[v[k] >> 22];
+        const bool open = (e.y >> 16) != 0 || v[k] == e.x;
+        const uint32_t byte = v[k] < e.x ? e.y & 255u : (e.y >> 8) & 255u;
+        bb |= (open ? 0 : byte) << (8 * k);
+        const unsigned m = __ballot_sync(FULL, open);
+        if (open) {
+          const int i = waiting + __popc(m & ((1u << lane) - 1u));
+          s_q[warp][i] = make_uint2(v[k], l[k]);
+          s_qid[warp][i] = (uint8_t)((q * 32 + lane) * 4 + k);
+        }
+        waiting += __popc(m);
+      }
+      wd[q] = bb;
+      while (waiting >= 32) {
+        bisect32(waiting - 32);
+        waiting -= 32;
+      }
+    }
+    bisect32(0);
+    waiting = 0;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const uint32_t bb = wd[q] | late[q * 32 + lane];
+      late[q * 32 + lane] = 0;
+      wd[q] = __funnelshift_l(bb, bb, rot[q]);
+    }
+    /* 64-bit word = (wd[0] << 32) | wd[1]; bit b = block b; the block of bit
+     * lane + 32 is two blocks up along z */
+    out[0] = warp_transpose32(wd[1], lane);
+    out[(int64_t)g.P / 2 * g.W] = warp_transpose32(wd[0], lane);
+    out += g.P * g.W;
   }
 }
 
@@ -1544,7 +1621,7 @@ k_from_ref(const micsa_geo g, const int p, const int ic, const int k,
     const uint64_t v = ref[h * g.nr + w * 32 + lane];
     const uint32_t lo = warp_transpose32((uint32_t)v, lane);
     const uint32_t hi = warp_transpose32((uint32_t)(v >> 32), lane);
-    const site_xyz a = ref_site(g, p, h, lane), b = ref_site(g, p, h, lane + 32);
+    const site_xyz a = ref_site(g, p, (uint32_t)h, lane), b = ref_site(g, p, (uint32_t)h, lane + 32);
     dst[demon_slot(g, p, ic, k, a.x, a.y, a.z) * g.W + w] = lo;
     dst[demon_slot(g, p, ic, k, b.x, b.y, b.z) * g.W + w] = hi;
   }
@@ -1584,7 +1661,7 @@ k_couplings_from_ref(const micsa_geo g, const uint64_t *__restrict__ J, uint8_t 
       if (d >= 3 && edge[d - 3]) w = rot_back_word(d, w);
       v |= (uint32_t)((w >> bit) & 1) << d;
     }
-    const site_xyz s = ref_site(g, p, h, bit);
+    const site_xyz s = ref_site(g, p, (uint32_t)h, bit);
     jb[(int64_t)p * g.P + ((int64_t)s.z * g.L + s.y) * g.Lh + (s.x >> 1)] = (uint8_t)v;
   }
 }
@@ -1599,7 +1676,7 @@ k_to_ref(const micsa_geo g, const int p, const int ic, const int *__restrict__ w
        wi += nwarps) {
     const int64_t h = wi / g.W;
     const int w = (int)(wi % g.W);
-    const site_xyz a = ref_site(g, p, h, lane), b = ref_site(g, p, h, lane + 32);
+    const site_xyz a = ref_site(g, p, (uint32_t)h, lane), b = ref_site(g, p, (uint32_t)h, lane + 32);
     const uint32_t lo = warp_transpose32(src[demon_slot(g, p, ic, k, a.x, a.y, a.z) * g.W + w], lane);
     const uint32_t hi = warp_transpose32(src[demon_slot(g, p, ic, k, b.x, b.y, b.z) * g.W + w], lane);
     ref[h * g.nr + w * 32 + lane] = (uint64_t)lo | ((uint64_t)hi << 32);
@@ -2192,10 +2269,32 @@ cudaError_t micsa_launch_sweep_metropolis(const micsa_geo &g, int p, uint32_t *s
   return sweep_any(g, p, 0, false, spin, nullptr, nullptr, jb, nullptr, rnd, nullptr, st);
 }
 
+void micsa_lut_bins(const void *lut, uint32_t *bins) {
+  const uint32_t *thr = (const uint32_t *)lut;
+  const uint16_t *pre = (const uint16_t *)((const uint8_t *)lut + 2048);
+  const uint32_t last = thr[2 * 254] >> 22;
+  for (uint32_t t = 0; t < 1024; t++) {
+    uint32_t a = pre[t] & 255u, b = pre[t] >> 8, open = t == last || b - a > 1;
+    if (t > last) a = b = 255, open = 0; /* above threshold 254 */
+    bins[2 * t] = thr[2 * a];
+    bins[2 * t + 1] = a | (b << 8) | (open << 16);
+  }
+}
+
 cudaError_t micsa_launch_gen_rnd(const micsa_geo &g, int p, const uint32_t *te,
                                  const uint32_t *keys, const uint8_t *lut, uint32_t *rnd,
                                  cudaStream_t st) {
-  k_gen_rnd<<<blocks_for(g.H * g.nr, TPB), TPB, 0, st>>>(g, p, te, keys, lut, rnd);
+  k_gen_rnd<rnd_arrays><<<blocks_for(g.H * g.nr, TPB), TPB, 0, st>>>(g, p, rnd_arrays{te, keys}, lut, rnd);
+  return cudaGetLastError();
+}
+
+cudaError_t micsa_launch_gen_rnd_values(const micsa_geo &g, int p, const uint32_t *te,
+                                        const uint32_t *keys, const uint8_t *lut, uint32_t *rnd,
+                                        cudaStream_t st) {
+  rnd_values v;
+  memcpy(v.te, te, 16 * (size_t)g.nr);
+  memcpy(v.keys, keys, 4 * (size_t)g.nr);
+  k_gen_rnd<rnd_values><<<blocks_for(g.H * g.nr, TPB), TPB, 0, st>>>(g, p, v, lut, rnd);
   return cudaGetLastError();
 }
 

@@ -136,10 +136,21 @@ cudaError_t micsa_launch_sweep_metropolis(const micsa_geo &g, int p,
                                           uint32_t *spin, const uint8_t *jb,
                                           const uint32_t *rnd, cudaStream_t st);
 /* Philox4x32-10 heat-bath words for colour p: te[r*4+k], keys[r] on device,
- * lut = 4096-byte table on device */
+ * lut = 4096-byte table on device, followed by its 8192 bytes of bin entries
+ * (micsa_lut_bins): per bin of a uniform's top 10 bits a threshold's high half,
+ * then the indices below and above it (8 bits each) and whether the bin needs
+ * the full search */
+#define MICSA_LUT_BYTES (4096 + 8192)
+void micsa_lut_bins(const void *lut, uint32_t *bins);
 cudaError_t micsa_launch_gen_rnd(const micsa_geo &g, int p, const uint32_t *te,
                                  const uint32_t *keys, const uint8_t *lut,
                                  uint32_t *rnd, cudaStream_t st);
+/* the same with te and keys on the host, for nr <= MICSA_RND_VALUES: they travel
+ * with the launch's arguments (at most 4 KB of them), no copy */
+#define MICSA_RND_VALUES 192
+cudaError_t micsa_launch_gen_rnd_values(const micsa_geo &g, int p, const uint32_t *te,
+                                        const uint32_t *keys, const uint8_t *lut,
+                                        uint32_t *rnd, cudaStream_t st);
 /* walk[s] = (walk[s] + 1) mod L/2 for all samples */
 cudaError_t micsa_launch_walk_advance(const micsa_geo &g, int *walk,
                                       cudaStream_t st);
