@@ -169,12 +169,12 @@ int ensure_stage(micsa_ctx *ctx) {
   return MICSA_OK;
 }
 
-/* The device address of a caller's host buffer that kernels may write
+/* The device address of a caller's host buffer that kernels may read and write
  * directly (page-locked and mapped, as cudaHostAlloc and mapped registered
- * memory are), else nullptr.  A download into such a buffer converts
- * straight into it across the host link: one pass at link speed instead of a
- * conversion into the staging buffer and then a copy. */
-uint64_t *device_view(uint64_t *p) {
+ * memory are), else nullptr.  Transfers from and to such a buffer convert
+ * straight across the host link: one pass at link speed instead of a copy
+ * and a conversion one after the other through the staging buffer. */
+uint64_t *device_view(const uint64_t *p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     (void)cudaGetLastError(); /* not a pointer the runtime knows: the staged path */
@@ -1074,16 +1074,20 @@ int micsa_upload_couplings(micsa_ctx *ctx, int sample, const uint64_t *J) {
 int micsa_upload_spins(micsa_ctx *ctx, int sample, const uint64_t *even, const uint64_t *odd) {
   if (!ctx || !even || !odd) return fail(ctx, MICSA_ERR_ARG, "null argument");
   int rc = check_sample(ctx, sample);
-  if (rc || (rc = set_device(ctx)) || (rc = ensure_stage(ctx))) return rc;
+  if (rc || (rc = set_device(ctx))) return rc;
   const micsa_geo &g = ctx->g;
   const int64_t n = g.H * g.nr;
-  MICSA_CK(cudaMemcpyAsync(ctx->stage, even, 8 * n, cudaMemcpyHostToDevice, ctx->stream));
-  MICSA_CK(cudaMemcpyAsync(ctx->stage + n, odd, 8 * n, cudaMemcpyHostToDevice, ctx->stream));
-  for (int p = 0; p < 2; p++) {
-    MICSA_CK(micsa_launch_from_ref(g, p, 0, 0, ctx->stage + p * n,
-                                   ctx->spin + ((int64_t)sample * 2 + p) * g.P * g.W, ctx->stream));
-    ctx->launches++;
+  const uint64_t *src[2] = {device_view(even), device_view(odd)};
+  if (!src[0] || !src[1]) {
+    if ((rc = ensure_stage(ctx))) return rc;
+    MICSA_CK(cudaMemcpyAsync(ctx->stage, even, 8 * n, cudaMemcpyHostToDevice, ctx->stream));
+    MICSA_CK(cudaMemcpyAsync(ctx->stage + n, odd, 8 * n, cudaMemcpyHostToDevice, ctx->stream));
+    src[0] = ctx->stage;
+    src[1] = ctx->stage + n;
   }
+  uint32_t *dst = ctx->spin + (int64_t)sample * 2 * g.P * g.W;
+  MICSA_CK(micsa_launch_from_ref(g, 1, 2, src[0], src[1], dst, dst + g.P * g.W, ctx->stream));
+  ctx->launches++;
   MICSA_CK(cudaStreamSynchronize(ctx->stream));
   ctx->have_spin[sample] = 1;
   return MICSA_OK;
@@ -1092,21 +1096,24 @@ int micsa_upload_spins(micsa_ctx *ctx, int sample, const uint64_t *even, const u
 int micsa_upload_demons(micsa_ctx *ctx, int sample, const uint64_t *w0, const uint64_t *w1) {
   if (!ctx || !w0 || !w1) return fail(ctx, MICSA_ERR_ARG, "null argument");
   int rc = check_sample(ctx, sample);
-  if (rc || (rc = set_device(ctx)) || (rc = ensure_stage(ctx))) return rc;
+  if (rc || (rc = set_device(ctx))) return rc;
   const micsa_geo &g = ctx->g;
-  const int64_t plane = g.H * g.nr, n = 2 * g.nc * plane;
-  const uint64_t *src[2] = {w0, w1};
-  uint32_t *dst[2] = {ctx->dem0, ctx->dem1};
-  for (int k = 0; k < 2; k++) {
-    MICSA_CK(cudaMemcpyAsync(ctx->stage, src[k], 8 * n, cudaMemcpyHostToDevice, ctx->stream));
-    for (int p = 0; p < 2; p++)
-      for (int ic = 0; ic < g.nc; ic++) {
-        const int64_t pi = (int64_t)p * g.nc + ic;
-        MICSA_CK(micsa_launch_from_ref(g, p, ic, 0, ctx->stage + pi * plane,
-                                       dst[k] + ((int64_t)sample * 2 * g.nc + pi) * g.P * g.W,
-                                       ctx->stream));
-        ctx->launches++;
-      }
+  const int planes = 2 * g.nc;
+  const int64_t n = planes * g.H * g.nr, o = (int64_t)sample * planes * g.P * g.W;
+  const uint64_t *src[2] = {device_view(w0), device_view(w1)};
+  if (src[0] && src[1]) {
+    MICSA_CK(micsa_launch_from_ref(g, planes, 2 * planes, src[0], src[1], ctx->dem0 + o, ctx->dem1 + o,
+                                   ctx->stream));
+    ctx->launches++;
+  } else { /* one array after the other through the staging buffer */
+    if ((rc = ensure_stage(ctx))) return rc;
+    const uint64_t *host[2] = {w0, w1};
+    uint32_t *dst[2] = {ctx->dem0 + o, ctx->dem1 + o};
+    for (int k = 0; k < 2; k++) {
+      MICSA_CK(cudaMemcpyAsync(ctx->stage, host[k], 8 * n, cudaMemcpyHostToDevice, ctx->stream));
+      MICSA_CK(micsa_launch_from_ref(g, planes, planes, ctx->stage, nullptr, dst[k], nullptr, ctx->stream));
+      ctx->launches++;
+    }
   }
   MICSA_CK(cudaMemsetAsync(ctx->walk + sample, 0, sizeof(int), ctx->stream));
   MICSA_CK(cudaStreamSynchronize(ctx->stream));
@@ -1492,17 +1499,17 @@ int micsa_measure(micsa_ctx *ctx, int32_t *e_spin, uint64_t *e_demon, int64_t *q
 int micsa_download_spins(micsa_ctx *ctx, int sample, uint64_t *even, uint64_t *odd) {
   if (!ctx || !even || !odd) return fail(ctx, MICSA_ERR_ARG, "null argument");
   int rc = check_sample(ctx, sample);
-  if (rc || (rc = set_device(ctx)) || (rc = ensure_stage(ctx))) return rc;
+  if (rc || (rc = set_device(ctx))) return rc;
   const micsa_geo &g = ctx->g;
   const int64_t n = g.H * g.nr;
   uint64_t *dv[2] = {device_view(even), device_view(odd)};
   const bool direct = dv[0] && dv[1];
-  for (int p = 0; p < 2; p++) {
-    MICSA_CK(micsa_launch_to_ref(g, p, 0, nullptr, sample,
-                                 ctx->spin + ((int64_t)sample * 2 + p) * g.P * g.W,
-                                 direct ? dv[p] : ctx->stage + p * n, ctx->stream));
-    ctx->launches++;
-  }
+  if (!direct && (rc = ensure_stage(ctx))) return rc;
+  const uint32_t *src = ctx->spin + (int64_t)sample * 2 * g.P * g.W;
+  MICSA_CK(micsa_launch_to_ref(g, 1, 2, nullptr, sample, src, src + g.P * g.W,
+                               direct ? dv[0] : ctx->stage, direct ? dv[1] : ctx->stage + n,
+                               ctx->stream));
+  ctx->launches++;
   if (!direct) {
     MICSA_CK(cudaMemcpyAsync(even, ctx->stage, 8 * n, cudaMemcpyDeviceToHost, ctx->stream));
     MICSA_CK(cudaMemcpyAsync(odd, ctx->stage + n, 8 * n, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1514,24 +1521,25 @@ int micsa_download_spins(micsa_ctx *ctx, int sample, uint64_t *even, uint64_t *o
 int micsa_download_demons(micsa_ctx *ctx, int sample, uint64_t *w0, uint64_t *w1) {
   if (!ctx || !w0 || !w1) return fail(ctx, MICSA_ERR_ARG, "null argument");
   int rc = check_sample(ctx, sample);
-  if (rc || (rc = set_device(ctx)) || (rc = ensure_stage(ctx))) return rc;
+  if (rc || (rc = set_device(ctx))) return rc;
   const micsa_geo &g = ctx->g;
-  const int64_t plane = g.H * g.nr, n = 2 * g.nc * plane;
-  const uint32_t *src[2] = {ctx->dem0, ctx->dem1};
+  const int planes = 2 * g.nc;
+  const int64_t n = planes * g.H * g.nr, o = (int64_t)sample * planes * g.P * g.W;
+  const uint32_t *src[2] = {ctx->dem0 + o, ctx->dem1 + o};
   uint64_t *dst[2] = {w0, w1};
   uint64_t *dv[2] = {device_view(w0), device_view(w1)};
-  const bool direct = dv[0] && dv[1];
-  for (int k = 0; k < 2; k++) {
-    for (int p = 0; p < 2; p++)
-      for (int ic = 0; ic < g.nc; ic++) {
-        const int64_t pi = (int64_t)p * g.nc + ic;
-        MICSA_CK(micsa_launch_to_ref(g, p, ic, ctx->walk, sample,
-                                     src[k] + ((int64_t)sample * 2 * g.nc + pi) * g.P * g.W,
-                                     (direct ? dv[k] : ctx->stage) + pi * plane, ctx->stream));
-        ctx->launches++;
-      }
-    if (!direct)
+  if (dv[0] && dv[1]) {
+    MICSA_CK(micsa_launch_to_ref(g, planes, 2 * planes, ctx->walk, sample, src[0], src[1], dv[0], dv[1],
+                                 ctx->stream));
+    ctx->launches++;
+  } else {
+    if ((rc = ensure_stage(ctx))) return rc;
+    for (int k = 0; k < 2; k++) {
+      MICSA_CK(micsa_launch_to_ref(g, planes, planes, ctx->walk, sample, src[k], nullptr, ctx->stage,
+                                   nullptr, ctx->stream));
+      ctx->launches++;
       MICSA_CK(cudaMemcpyAsync(dst[k], ctx->stage, 8 * n, cudaMemcpyDeviceToHost, ctx->stream));
+    }
   }
   MICSA_CK(cudaStreamSynchronize(ctx->stream));
   return MICSA_OK;

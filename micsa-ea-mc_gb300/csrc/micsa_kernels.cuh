@@ -157,21 +157,20 @@ cudaError_t micsa_launch_walk_advance(const micsa_geo &g, int *walk,
 /* walk[s] = (walk[s] + n) mod L/2 for the running samples */
 cudaError_t micsa_launch_walk_add(const micsa_geo &g, int *walk, int n, cudaStream_t st);
 
-/* reference-layout words ref[h*nr + r] (one colour, one sample/plane) ->
- * device words dst (colour p base of that plane), demon translation k
- * (0 for spins) applied with plane index ic (ignored when k == 0) */
-cudaError_t micsa_launch_from_ref(const micsa_geo &g, int p, int ic, int k,
-                                  const uint64_t *ref, uint32_t *dst,
+/* reference-layout planes (ref[h*nr + r] each) -> device planes and back, in one
+ * launch: `planes` planes, the first `first` of them from ref0 to dst0, the
+ * rest from ref1 to dst1 (spins: first = 1, planes = 2; demons: first = 2nc).
+ * The reference arrays may be mapped host memory. */
+cudaError_t micsa_launch_from_ref(const micsa_geo &g, int first, int planes, const uint64_t *ref0,
+                                  const uint64_t *ref1, uint32_t *dst0, uint32_t *dst1,
                                   cudaStream_t st);
+cudaError_t micsa_launch_to_ref(const micsa_geo &g, int first, int planes, const int *walk,
+                                int sample, const uint32_t *src0, const uint32_t *src1,
+                                uint64_t *ref0, uint64_t *ref1, cudaStream_t st);
 /* reference coupling words J[(p*6 + d)*H + h] of one sample (device) ->
  * that sample's bond bytes jb[2][P] */
 cudaError_t micsa_launch_couplings_from_ref(const micsa_geo &g, const uint64_t *J, uint8_t *jb,
                                             cudaStream_t st);
-cudaError_t micsa_launch_to_ref(const micsa_geo &g, int p, int ic,
-                                const int *walk, int sample,
-                                const uint32_t *src, uint64_t *ref,
-                                cudaStream_t st);
-
 /* measurement accumulators (unsigned long long, zeroed by the caller):
  *   unsat[s*nr + r], dem[s*nr + r], qd[s*(nr/2) + k],
  *   c4d[((s*(nr/2) + k)*3 + axis)*(L/2+1) + d] */
