@@ -216,19 +216,20 @@ int micsa_profile(micsa_ctx *ctx, int64_t n, double *sweep_ms, double *iteration
  * persistent form, as many blocks as fit the GPU, each looping over tickets
  * and taking the next during its tile | quad: direct loads with
  * four one-word sites per thread (32 replicas)>
- * tile=<default | row: blocks span whole rows along x>[/2: half-height
+ * tile=<default | row: blocks span whole rows along x | lin, lin4: blocks of
+ * consecutive units of two or four sites (flow)>[/2: half-height
  * dataflow tiles]
  * fit=<iterations per launch of the dataflow sweep: its wavefront runs on
  * from one iteration into the next; 1 for the other loads>
  * chains=<K: the samples' launches in K chains side by side>/<iterations per
  * graph replay> |
- * <zc>/<pd>/<split>/<occ>/<load 0|1|2|3|4|5|6 (6: pflow)>/<tile 0|1>:<ms per half-sweep> ...",
+ * <zc>/<pd>/<split>/<occ>/<load 0|1|2|3|4|5|7 (4: flow, 7: flow with quads)>/<tile 0|1|2>:<ms per half-sweep> ...",
  * with " cached" before the "|" when the choice and its table were taken
  * over from an earlier context of the same device, L, nr, samples and nc in
  * this process (MICSA_TUNE_CACHE=0 times every context instead).  The
  * environment variables MICSA_SWEEP_ZC, MICSA_SWEEP_PD, MICSA_SWEEP_SPLIT,
  * MICSA_SWEEP_OCC, MICSA_SWEEP_TMA, MICSA_SWEEP_ASYNC, MICSA_SWEEP_PIPE,
- * MICSA_SWEEP_FLOW, MICSA_SWEEP_QUAD and MICSA_SWEEP_TILE (=row), read by
+ * MICSA_SWEEP_FLOW, MICSA_SWEEP_QUAD and MICSA_SWEEP_TILE (=row, or =lin with the dataflow sweep), read by
  * micsa_create, pin the shape and skip the timing (no candidates listed
  * then).  The dataflow sweep is timed for L >= 128 only; MICSA_SWEEP_FLOW=0
  * alone leaves it out everywhere.  The reference has fixed launch geometry
@@ -293,7 +294,7 @@ int64_t micsa_job_measurements(int64_t iterations);
 /* Run njobs jobs together.  Jobs of one shape (L, nr, nc, beta) share a
  * context, one job per sample slot, longest first; each shape group runs in
  * its own context and stream on `device`, concurrently with the others.  In
- * a group one launch per half-sweep (or per 1024 iterations at L <= 16),
+ * a group one launch per half-sweep (or per 1024 iterations at L <= 32),
  * refresh and measurement serves every running job; a job whose iterations
  * are done is frozen (micsa_set_active) after its last measurement.
  * Outputs (either may be NULL), m = measurement point, nm_j =

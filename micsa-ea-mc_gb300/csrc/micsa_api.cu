@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "micsa.h"
+#include "micsa_internal.h"
 #include "micsa_jump.h"
 #include "micsa_kernels.cuh"
 
@@ -31,6 +32,7 @@
 struct micsa_ctx {
   micsa_config cfg;
   micsa_geo g;
+  bool shared = false; /* one of several contexts that run side by side */
   cudaStream_t stream = nullptr;
   uint32_t *spin = nullptr, *dem0 = nullptr, *dem1 = nullptr, *rnd = nullptr;
   uint8_t *jb = nullptr, *lut = nullptr;
@@ -311,7 +313,7 @@ cudaError_t ensure_chains(micsa_ctx *ctx, int K) {
 }
 
 /* Launch shapes chosen so far in this process, by (device, L, nr, samples,
- * nc, TMA maps usable): a context of a shape timed before takes the earlier
+ * nc, TMA maps usable, side by side with others or alone): a context of a shape timed before takes the earlier
  * choice and table instead of timing again, so batches and servers that open
  * many contexts of a few shapes pay for each shape once. */
 struct tune_entry {
@@ -320,11 +322,11 @@ struct tune_entry {
   std::vector<double> ms;
 };
 std::mutex tune_mu;
-std::map<std::tuple<int, int, int, int, int, int>, tune_entry> tune_cache;
+std::map<std::tuple<int, int, int, int, int, int, bool>, tune_entry> tune_cache;
 
-std::tuple<int, int, int, int, int, int> tune_key(const micsa_ctx *ctx) {
+std::tuple<int, int, int, int, int, int, bool> tune_key(const micsa_ctx *ctx) {
   return std::make_tuple(ctx->cfg.device, ctx->g.L, ctx->cfg.nr, ctx->g.ns, ctx->g.nc,
-                         ctx->tma.ok ? 1 : 0);
+                         ctx->tma.ok ? 1 : 0, ctx->shared);
 }
 
 /* Launch-shape autotuner: time whole iterations (the half-sweeps in their
@@ -340,6 +342,8 @@ int autotune(micsa_ctx *ctx) {
   micsa_geo &g = ctx->g;
   int zcs[8];
   const int nz = micsa_sweep_zc_candidates(g.L, zcs, 8);
+  int fzcs[16]; /* slab depths of the dataflow sweep */
+  const int nfz = micsa_flow_zc_candidates(g.L, fzcs, 16);
   const int pds[3] = {0, 2, 4};
   /* MICSA_SWEEP_ZC / MICSA_SWEEP_PD pin the shape and skip the timing
    * (reproducible launch shapes, e.g. under a profiler, whose per-launch
@@ -349,6 +353,8 @@ int autotune(micsa_ctx *ctx) {
     const int zc = atoi(ez), pd = ep ? atoi(ep) : 0;
     int ok = 0;
     for (int c = 0; c < nz; c++) ok |= zcs[c] == zc;
+    if (const char *ef = getenv("MICSA_SWEEP_FLOW"))
+      for (int c = 0; c < nfz && atoi(ef); c++) ok |= fzcs[c] == zc;
     if (!ok || (pd != 0 && pd != 2 && pd != 4) || (pd && pd >= zc))
       return fail(ctx, MICSA_ERR_ARG, "MICSA_SWEEP_ZC=%d / MICSA_SWEEP_PD=%d not a shape for L=%d",
                   zc, pd, g.L);
@@ -364,11 +370,13 @@ int autotune(micsa_ctx *ctx) {
     g.pipe = ep2 && atoi(ep2) && !g.tma && !g.async;
     g.tw = ew && !strcmp(ew, "row") && !g.tma && micsa_sweep_wide_differs(g.L, eq && atoi(eq) ? 4 : 2);
     g.flow = ef && atoi(ef) && !g.tma && !g.async && !g.pipe;
-    g.quad = eq && atoi(eq) && g.W == 1 && !g.tma && !g.async && !g.pipe && !g.flow;
     if (const char *ep = getenv("MICSA_SWEEP_PERS")) g.pers = g.flow && atoi(ep) == 1;
-    if (const char *eh = getenv("MICSA_FLOW_HALF")) g.half = g.flow && !g.pers && atoi(eh) == 1;
+    if (g.flow && !g.pers && ew && !strcmp(ew, "lin")) g.tw = 2;
+    g.quad = eq && atoi(eq) && g.W == 1 && !g.tma && !g.async && !g.pipe && (!g.flow || g.tw == 2);
+    if (const char *eh = getenv("MICSA_FLOW_HALF"))
+      g.half = g.flow && !g.pers && g.tw != 2 && atoi(eh) == 1;
     if (const char *ex = getenv("MICSA_FLOW_XS"))
-      g.xs = g.flow && !g.pers && !g.half && atoi(ex) == 1;
+      g.xs = g.flow && !g.pers && !g.half && g.tw != 2 && atoi(ex) == 1;
     if (const char *ek = getenv("MICSA_FLOW_ITERS")) {
       const int k = atoi(ek);
       if (g.flow && k >= 1 && k <= 64) g.fit = k;
@@ -429,19 +437,22 @@ int autotune(micsa_ctx *ctx) {
   MICSA_CK(cudaEventCreate(&e1));
   double best = 1e30;
   int best_zc = zcs[nz - 1], best_pd = 0, best_split = 0, best_occ = 3, best_tma = 0;
-  int best_async = 0, best_pipe = 0, best_tw = 0, best_flow = 0, best_quad = 0, best_pers = 0;
+  int best_async = 0, best_pipe = 0, best_tw = 0, best_flow = 0, best_quad = 0;
   int n = 0;
   const int ntw = micsa_sweep_wide_differs(g.L) ? 2 : 1, ntw4 = micsa_sweep_wide_differs(g.L, 4) ? 2 : 1;
-  /* The dataflow sweep is timed only for large lattices (many slabs per
-   * half-sweep, so that its tiles rarely wait): contexts of small lattices
-   * run side by side in batches and servers, where blocks that wait on
-   * dependencies hold SM slots the other contexts' kernels need (the batched
-   * mixed-L stream lost 30% with it).  Alone it loses as well below L=128,
-   * where a half-sweep has too few slabs for tiles to find work ahead (L=64 x 8
-   * samples: 1.30 against 7.02 attempts/ps; L=96 x 16: 3.85 against 6.75).
-   * MICSA_SWEEP_FLOW=0 leaves it out everywhere. */
+  /* The contexts of a batch's groups and of a server's pools run side by
+   * side, where blocks that wait for a slab hold SM slots the other contexts'
+   * kernels need: with the dataflow sweep at every size the served stream
+   * fell from 5.41 to 4.66 anneals/s and the batched one from 92.6 to 87.7.
+   * Theirs try it only for L >= 128 (where they would run few samples); a
+   * context of its own tries it at every L (us per iteration, against the
+   * best of the other forms: L=64, 8 samples x 64 replicas 87 against 102;
+   * L=96, 2 x 64: 84 against 99; L=104, 3 x 32: 103 against 123; L=48,
+   * 32 x 64: 143 against 151).  MICSA_SWEEP_FLOW=0 leaves it out everywhere. */
   const char *ef0 = getenv("MICSA_SWEEP_FLOW");
-  const bool try_flow = !(ef0 && !strcmp(ef0, "0")) && g.L >= 128;
+  const bool try_flow = !(ef0 && !strcmp(ef0, "0")) && (g.L >= 128 || !ctx->shared);
+  int nsm = 0;
+  MICSA_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->cfg.device));
   const int reps = 3;
   /* sample orders: all samples per launch, or sample-major.  Launches per
    * group of 2 to 8 samples (MICSA_SWEEP_SPLIT=k) are not timed: alone they
@@ -488,28 +499,40 @@ int autotune(micsa_ctx *ctx) {
     return MICSA_OK;
   };
   int rc = MICSA_OK;
-  for (int tm = 0; tm < 7; tm++)
-  for (int tw = 0; tw < (tm == 5 ? ntw4 : ntw); tw++)
+  for (int tm : {0, 1, 2, 3, 4, 5, 7})
+  for (int tw = 0; tw < (tm == 4 || tm == 7 ? 1 : (tm == 5 ? ntw4 : ntw)); tw++)
   for (int oc = 0; oc < nocc; oc++)
   for (int si = 0; si < nsp; si++)
-  for (int c = 0; c < nz; c++)
+  for (int c = 0; c < (tm == 4 || tm == 7 ? nfz : nz); c++)
     for (int d = 0; d < 3; d++) {
-      if (pds[d] && pds[d] >= zcs[c]) continue; /* prefetch only within a slab */
-      if (tm == 1 && (!ctx->tma.ok || zcs[c] > 4)) continue; /* staged tiles: <= 4 planes */
+      const int zc = tm == 4 || tm == 7 ? fzcs[c] : zcs[c];
+      if (pds[d] && pds[d] >= zc) continue; /* prefetch only within a slab */
+      if (tm == 1 && (!ctx->tma.ok || zc > 4)) continue; /* staged tiles: <= 4 planes */
       if (tm == 2 && (g.W != 2 || pds[d])) continue;          /* no L2 prefetch there */
       if (tw && (tm == 1 || tm == 2)) continue; /* whole-row blocks: direct and pipelined loads */
-      if (((tm == 4 || tm == 6) && !try_flow) || (tm == 5 && g.W != 1)) continue;
+      if (((tm == 4 || tm == 7) && !try_flow) || ((tm == 5 || tm == 7) && g.W != 1)) continue;
       const int sp = sps[si];
-      g.zc = zcs[c];
+      if (tm == 4 || tm == 7) {
+        /* tiles of a half-sweep (of one sample in sample-major order) against
+         * the blocks the GPU holds: with fewer the tiles wait for each other,
+         * with more of them than need be their prologues cost more -- the
+         * fastest depth had 0.84 (L=64, 8 samples) to 1.3 (L=160) of the
+         * blocks at all sizes tried, so the others are not timed */
+        const double tiles = (double)((g.L * g.Lh / (tm == 7 ? 4 : 2) + 255) / 256) *
+                             (g.W % 4 == 0 ? g.W / 4 : (g.W % 2 == 0 ? g.W / 2 : g.W)) * (g.L / zc) * (sp ? 1 : g.ns);
+        const double held = (double)nsm * (g.W % 4 ? (oc ? 4 : 3) : 2);
+        const bool last = c + 1 == nfz;
+        if (tiles < 0.7 * held || (tiles > 2.2 * held && !last)) continue;
+      }
+      g.zc = zc;
       g.pd = pds[d];
       g.occ = tm == 3 ? (oc ? 2 : 3) : (oc ? 4 : 3);
       g.tma = tm == 1;
       g.async = tm == 2;
       g.pipe = tm == 3;
-      g.tw = tw;
-      g.flow = tm == 4 || tm == 6;
-      g.pers = tm == 6;
-      g.quad = tm == 5;
+      g.flow = tm == 4 || tm == 7;
+      g.tw = g.flow ? 2 : tw;
+      g.quad = tm == 5 || tm == 7;
       /* the dataflow sweep is timed carrying 16 iterations per launch, its
        * best form (the launch boundary drains the GPU); the count is
        * settled below for the chosen shape */
@@ -526,7 +549,7 @@ int autotune(micsa_ctx *ctx) {
         ctx->tune_split[n] = sp;
         ctx->tune_occ[n] = g.occ;
         ctx->tune_load[n] = tm;
-        ctx->tune_tw[n] = tw;
+        ctx->tune_tw[n] = g.tw;
         ctx->tune_ms[n] = per;
         n++;
       }
@@ -541,7 +564,6 @@ int autotune(micsa_ctx *ctx) {
         best_pipe = g.pipe;
         best_tw = g.tw;
         best_flow = g.flow;
-        best_pers = g.pers;
         best_quad = g.quad;
       }
     }
@@ -572,9 +594,8 @@ int autotune(micsa_ctx *ctx) {
         g.async = tm == 2;
         g.pipe = tm == 3;
         g.tw = ctx->tune_tw[c];
-        g.flow = tm == 4 || tm == 6;
-        g.pers = tm == 6;
-        g.quad = tm == 5;
+        g.flow = tm == 4 || tm == 7;
+        g.quad = tm == 5 || tm == 7;
         g.fit = g.flow ? 16 : 1;
         double per = 0;
         if ((rc = time_shape(ctx->tune_split[c], 3 * reps, &per))) return rc;
@@ -589,7 +610,6 @@ int autotune(micsa_ctx *ctx) {
           best_pipe = g.pipe;
           best_tw = g.tw;
           best_flow = g.flow;
-          best_pers = g.pers;
           best_quad = g.quad;
         }
       }
@@ -605,7 +625,6 @@ int autotune(micsa_ctx *ctx) {
   g.pipe = best_pipe;
   g.tw = best_tw;
   g.flow = best_flow;
-  g.pers = best_pers;
   g.quad = best_quad;
   g.fit = 1;
   double best_flow_it = 1e30;
@@ -642,37 +661,6 @@ int autotune(micsa_ctx *ctx) {
       if (per < best_it) best_it = per, best_fit = k;
     }
     g.fit = best_fit;
-    if (!g.pers) {
-      /* half-height tiles: twice the tiles per slab, each half as long, for a
-       * sweep whose wavefront of dependencies bounds it */
-      g.half = 1;
-      cudaGraph_t gr = nullptr;
-      cudaGraphExec_t ge = nullptr;
-      MICSA_CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-      cudaError_t le = launch_halves(ctx, g, ctx->split, 0, g.nc, nullptr);
-      if (le == cudaSuccess)
-        le = g.fit > 1 ? micsa_launch_walk_add(g, ctx->walk, g.fit, ctx->stream)
-                       : micsa_launch_walk_advance(g, ctx->walk, ctx->stream);
-      const cudaError_t ce = cudaStreamEndCapture(ctx->stream, &gr);
-      MICSA_CK(le);
-      MICSA_CK(ce);
-      const cudaError_t ie = cudaGraphInstantiate(&ge, gr, 0);
-      cudaGraphDestroy(gr);
-      MICSA_CK(ie);
-      const int rr = g.fit >= 16 ? 1 : (g.fit >= 4 ? 2 : 6);
-      float ms = 0;
-      cudaError_t te = cudaGraphLaunch(ge, ctx->stream);
-      if (te == cudaSuccess) te = cudaEventRecord(e0, ctx->stream);
-      for (int rep = 0; rep < rr && te == cudaSuccess; rep++) te = cudaGraphLaunch(ge, ctx->stream);
-      if (te == cudaSuccess) te = cudaEventRecord(e1, ctx->stream);
-      if (te == cudaSuccess) te = cudaEventSynchronize(e1);
-      if (te == cudaSuccess) te = cudaEventElapsedTime(&ms, e0, e1);
-      cudaGraphExecDestroy(ge);
-      MICSA_CK(te);
-      const double hit = ms / ((double)rr * g.fit);
-      if (hit >= best_it) g.half = 0;
-      else best_it = hit;
-    }
     best_flow_it = best_it;
   }
   /* Samples in chains side by side, and several iterations per graph replay,
@@ -687,7 +675,7 @@ int autotune(micsa_ctx *ctx) {
     if (g.flow) base = best_flow_it;
     int two[2], nt = 0;
     for (int c = 0; c < n && c < MICSA_TUNE_MAX; c++) {
-      if (ctx->tune_load[c] == 4 || ctx->tune_load[c] == 6 || ctx->tune_split[c]) continue;
+      if (ctx->tune_load[c] == 4 || ctx->tune_load[c] == 7 || ctx->tune_split[c]) continue;
       if (nt < 2) two[nt++] = c;
       else if (ctx->tune_ms[c] < ctx->tune_ms[two[1]]) two[1] = c;
       if (nt == 2 && ctx->tune_ms[two[1]] < ctx->tune_ms[two[0]]) std::swap(two[0], two[1]);
@@ -844,7 +832,8 @@ int64_t micsa_footprint_bytes(const micsa_config *cfg) {
          4 * (9 * (int64_t)cfg->nr) + 4 * MICSA_MAX_SAMPLES;
 }
 
-int micsa_create(const micsa_config *cfg, micsa_ctx **out) {
+namespace {
+int create_ctx(const micsa_config *cfg, bool shared, micsa_ctx **out) {
   if (!out) return MICSA_ERR_ARG;
   *out = nullptr;
   char msg[256];
@@ -856,6 +845,7 @@ int micsa_create(const micsa_config *cfg, micsa_ctx **out) {
   micsa_ctx *ctx = new (std::nothrow) micsa_ctx();
   if (!ctx) return MICSA_ERR_NOMEM;
   ctx->cfg = *cfg;
+  ctx->shared = shared;
   sizes s = sizes_of(*cfg);
   micsa_geo &g = ctx->g;
   g.L = cfg->L;
@@ -966,13 +956,18 @@ int micsa_create(const micsa_config *cfg, micsa_ctx **out) {
 #undef MICSA_CK_CREATE
   return MICSA_OK;
 }
+}  // namespace
+
+int micsa_create(const micsa_config *cfg, micsa_ctx **out) { return create_ctx(cfg, false, out); }
+
+int micsa_create_shared(const micsa_config *cfg, micsa_ctx **out) { return create_ctx(cfg, true, out); }
 
 int micsa_tuning_report(const micsa_ctx *ctx, char *buf, size_t n) {
   if (!ctx || !buf || n == 0) return MICSA_ERR_ARG;
   int k = snprintf(buf, n, "zc=%d pd=%d split=%d occ=%d load=%s tile=%s%s%s fit=%d chains=%d/%d%s |", ctx->g.zc,
                    ctx->g.pd, ctx->split, ctx->g.occ,
                    ctx->g.tma ? "tma" : (ctx->g.async ? "async" : (ctx->g.pipe ? "pipe" : (ctx->g.flow ? (ctx->g.pers ? "pflow" : "flow") : (ctx->g.quad ? "quad" : "direct")))),
-                   ctx->g.tw ? "row" : "default", ctx->g.flow && ctx->g.half ? "/2" : "",
+                   ctx->g.tw == 2 ? (ctx->g.quad ? "lin4" : "lin") : ctx->g.tw ? "row" : "default", ctx->g.flow && ctx->g.half ? "/2" : "",
                    ctx->g.flow && ctx->g.xs ? "+xs" : "",
                    ctx->g.flow ? ctx->g.fit : 1, ctx->g.flow || ctx->split ? 1 : ctx->chains,
                    ctx->g.flow ? ctx->g.fit : ctx->unit,

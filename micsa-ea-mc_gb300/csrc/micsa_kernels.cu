@@ -669,9 +669,9 @@ k_sweep(const micsa_geo g, const int p, const int ic, const int ytiles, const in
  * slab) * j.  Tiles wait only on earlier tickets, and a ticket is only held
  * by a running block, so the earliest unfinished tile can always run: the
  * launch needs no co-residency.  The lead thread polls the three counters
- * with relaxed loads issued together, then an acquire fence and a block
- * barrier order the tile's loads after the producers' stores; a producer
- * releases with a block barrier, a fence and an atomic add.  Waits are
+ * (first warp) polls the three counters with acquire loads, one lane each,
+ * and a block barrier orders the tile's loads after the producers' stores; a
+ * producer releases with the last of its warps' additions.  Waits are
  * bounded (2 s by the global timer; after one runs out every later wait
  * gives up at once, and micsa_flow_timeouts counts them); the last block to
  * finish resets the counters for the next launch. */
@@ -712,9 +712,40 @@ __device__ __forceinline__ bool flow_wait3(const unsigned *a, const unsigned *b,
   return ok;
 }
 
-/* The lead thread's part: take a ticket, decode it into job[] (s, j, slab,
- * bx, row tile, group, walk) from the launch's constants in cst[] and wait
- * for the tile's dependencies. */
+__device__ __forceinline__ unsigned add_acq_rel_cta(unsigned *a, unsigned v) {
+  unsigned o;
+  asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;"
+               : "=r"(o) : "r"(smem_addr(a)), "r"(v) : "memory");
+  return o;
+}
+
+__device__ __forceinline__ void red_release_gpu(unsigned *a, unsigned v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(a), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *a) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+  return v;
+}
+/* the same by one warp, a counter per lane: each lane acquires its own, so no
+ * fence follows; ok holds the result of a first look, and a lane with need 0
+ * has nothing to wait for */
+__device__ __forceinline__ void flow_wait_lanes(const unsigned *c, unsigned need, bool ok) {
+  for (uint64_t t0 = 0; !__all_sync(FULL, ok);) {
+    if (!t0) t0 = global_ns();
+    if (*(volatile unsigned *)&micsa_flow_timeouts || global_ns() - t0 > micsa_flow_limit_ns) {
+      if (!ok) atomicAdd(&micsa_flow_timeouts, 1u);
+      ok = true;
+      continue;
+    }
+    __nanosleep(64);
+    if (!ok) ok = ld_acquire_u32(c) >= need;
+  }
+}
+
+/* The persistent form's lead thread: decode a ticket into job[] (s, j, slab,
+ * bx, row tile, group, walk) by the launch's constants in cst[] ... */
 enum { C_GX, C_NSLAB, C_T, C_PER_HALF, C_PER_SAMPLE, C_YT, C_SMAJ, C_N };
 __device__ __forceinline__ void dep_decode(const micsa_geo &g, const int *__restrict__ walk,
                                            const unsigned *cst, const unsigned u, unsigned *job) {
@@ -739,11 +770,6 @@ __device__ __forceinline__ void dep_decode(const micsa_geo &g, const int *__rest
   job[4] = (t / gx) % ytiles;
   job[5] = t / (gx * ytiles);
   job[6] = (unsigned)__ldg(walk + s);
-}
-__device__ __forceinline__ void dep_take(const micsa_geo &g, const int *__restrict__ walk,
-                                         unsigned *__restrict__ ctl, const unsigned *cst,
-                                         unsigned *job) {
-  dep_decode(g, walk, cst, atomicAdd(ctl, 1u), job);
 }
 /* ... and the lead thread's wait for the tile's dependencies */
 __device__ __forceinline__ void dep_wait(const micsa_geo &g, unsigned *__restrict__ ctl,
@@ -795,79 +821,138 @@ __device__ __forceinline__ void prefetch_tile_demons(const micsa_geo &g, int p, 
   }
 }
 
-/* The tile's values go through shared memory and are read where they are
+/* n / d for n < 2^31 by one multiplication: m = ceil(2^(31+sh) / d) with
+ * 2^sh >= d, whose error stays below one quotient for such n */
+struct micsa_udiv {
+  unsigned d, m, sh;
+  __host__ explicit micsa_udiv(unsigned d_) : d(d_), sh(0) {
+    while ((1ull << sh) < d) sh++;
+    m = (unsigned)(((1ull << (31 + sh)) + d - 1) / d);
+  }
+  __device__ __forceinline__ unsigned operator()(unsigned n) const {
+    return (unsigned)(((uint64_t)n * m) >> (31 + sh));
+  }
+};
+/* the launch's constants, by which a ticket is decoded: tickets per sample
+ * (sample-major) or per half-sweep of all samples, tiles per half-sweep of a
+ * sample, per slab, per row of tiles and per word group; slabs; half-sweeps
+ * of an iteration; units of a row (LIN) */
+struct micsa_flow_plan {
+  micsa_udiv outer, half, slab, gx, yt, nslab, per_it, pairs;
+  int smaj;
+};
+
+/* One tile per block.  Neither DRAM (58% of its peak at L=160) nor the ALU
+ * pipe bounds it, but the time a tile spends beside its z loop: the chain of
+ * round trips before any warp can load, and the one after the last store
+ * before its slot is free again (9600 of a tile's 28600 cycles at L=160, 8
+ * planes).  So both are kept short: the ticket is decoded by multiplications
+ * instead of divisions; the sample's walk, its run flag and the three slab
+ * counters are loaded together, a lane each, by acquire loads that no fence
+ * follows; the last warp to finish adds to the slab counter with a release,
+ * without a block barrier, and nothing waits for the addition; and the
+ * counters are cleared after the launch, not by a last block that every
+ * block would have to look for.  With tiles that cost less apart from their
+ * planes, thinner slabs pay (L=160: 5 planes, 1.3 times as many tiles a
+ * half-sweep as the GPU holds, where 8 planes had 0.8 and waited).  L=160, 2
+ * samples x 64 replicas, us per iteration: 378 before, 344 so.  A persistent
+ * form with a control warp that takes the next ticket during a tile was no
+ * faster (370): the tickets it holds ahead widen the window in flight, and
+ * its tiles wait for slabs instead.
+ *
+ * LIN: the block takes TPB consecutive (row, x/2) units of S sites of the
+ * slab's planes instead of a rectangle of rows: as coalesced as whole rows,
+ * and no idle lanes where a row's units do not divide the block (L=160: 25
+ * tiles a slab of 8 full warps instead of 27 of 7.5; 386 -> 371 us at 8
+ * planes).  Four one-word sites a thread (S = 4) halve the tiles of
+ * 32-replica lattices (L=104, 3 samples: 106 us, 110 by pairs; L=128, 1
+ * sample: 73, 78 by pairs).
+ *
+ * The tile's values go through shared memory and are read where they are
  * used, so that none of them stays in a register across the sweep body
  * (which needs about all of the 64 registers of the 4-blocks budget). */
-template <int VW, bool WIDE, int MINB, int BT = TPB, bool XS = false>
+template <int VW, bool WIDE, int MINB, int BT = TPB, bool XS = false, bool LIN = false, int S = 2>
 __global__ void __launch_bounds__(BT, MINB)
-k_sweep_dep(const __grid_constant__ micsa_geo g, const int ytiles, const int G, const int zc,
-            const int pd, const int smaj, const int pf, uint32_t *__restrict__ spin,
-            uint32_t *__restrict__ d0,
-            uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb,
-            const int *__restrict__ walk, unsigned *__restrict__ ctl) {
+k_sweep_dep(const __grid_constant__ micsa_geo g, const __grid_constant__ micsa_flow_plan f,
+            const int zc, const int pd, const int pf, uint32_t *__restrict__ spin,
+            uint32_t *__restrict__ d0, uint32_t *__restrict__ d1,
+            const uint8_t *__restrict__ jb, const int *__restrict__ walk,
+            unsigned *__restrict__ ctl) {
   /* the z loop unrolled once where two steps' registers do not fit: pairs
    * of two-word sites at 64 registers per thread (16-byte spills against 32
    * unrolled twice; L=160: 8.34 against 8.16 attempts/ps) and the shuffle
    * form (which spills unrolled twice at 80) */
   constexpr int UNR = (XS || (VW >= 2 && 65536 / (MINB * BT) <= 64)) ? 1 : 2;
+  enum { J_S, J_HALF, J_SLAB, J_X, J_Y, J_GRP, J_WALK, J_RUN, J_N };
+  __shared__ unsigned job[J_N], done;
+  const unsigned lin = threadIdx.y * blockDim.x + threadIdx.x;
+  /* first warp: lane 0 takes the ticket; lanes 0-2 hold a slab counter each,
+   * lane 3 the walk, lane 4 the run flag, in one round trip */
+  unsigned need = 0, v = 0;
+  const unsigned *c = nullptr;
+  bool ok = true;
   grid_dependency_sync();
-  __shared__ unsigned cst[C_N];
-  __shared__ unsigned job[8]; /* s, j, slab, bx, row tile, group, walk, last */
-  const bool lead = threadIdx.x == 0 && threadIdx.y == 0;
-  if (lead) {
-    const unsigned gx = (unsigned)g.Lh / 2u / blockDim.x; /* blocks along x */
-    const unsigned nslab = (unsigned)(g.L / zc);
-    const unsigned T = gx * (unsigned)ytiles * (unsigned)G; /* tiles per slab */
-    cst[C_GX] = gx;
-    cst[C_NSLAB] = nslab;
-    cst[C_T] = T;
-    cst[C_YT] = (unsigned)ytiles;
-    cst[C_PER_HALF] = nslab * T;
-    cst[C_PER_SAMPLE] = (unsigned)(g.fit > 1 ? g.fit : 1) * 2u * (unsigned)g.nc * nslab * T;
-    cst[C_SMAJ] = (unsigned)smaj;
-    dep_take(g, walk, ctl, cst, job);
-    if (pf <= 0) dep_wait(g, ctl, cst, job);
+  if (lin < 32u) {
+    if (lin == 0) v = atomicAdd(ctl, 1u);
+    const unsigned u = __shfl_sync(FULL, v, 0);
+    const unsigned a = f.outer(u), r = u - a * f.outer.d, h = f.half(r), r2 = r - h * f.half.d;
+    const unsigned s = f.smaj ? a : h, j = f.smaj ? h : a, q = f.slab(r2), t = r2 - q * f.slab.d;
+    unsigned b = q + (j - f.nslab(j) * f.nslab.d);
+    b -= b >= f.nslab.d ? f.nslab.d : 0;
+    unsigned bl = b + (lin == 2u) - (lin == 0u); /* slabs b-1, b, b+1 around the lattice */
+    bl = bl == f.nslab.d ? 0 : (bl == ~0u ? f.nslab.d - 1 : bl);
+    c = ctl + 4 + s * f.nslab.d + bl;
+    if (lin < 3u) v = ld_acquire_u32(c);
+    else if (lin == 3u) v = (unsigned)__ldg(walk + s);
+    else if (lin == 4u) v = !micsa_frozen(g, (int)s);
+    const unsigned w = __shfl_sync(FULL, v, 3), run = __shfl_sync(FULL, v, 4);
+    need = run && j > 0 && lin < 3u ? f.slab.d * j + micsa_flow_need_offset : 0u;
+    ok = v >= need;
+    if (lin == 0) {
+      const unsigned it = f.per_it(j), tx = f.gx(t), ty = f.yt(tx);
+      job[J_S] = s;
+      job[J_HALF] = j - it * f.per_it.d;
+      job[J_SLAB] = b;
+      job[J_X] = t - tx * f.gx.d;
+      job[J_Y] = tx - ty * f.yt.d;
+      job[J_GRP] = ty;
+      job[J_WALK] = w + it;
+      job[J_RUN] = run;
+      done = 0;
+    }
+    if (pf <= 0) flow_wait_lanes(c, need, ok);
   }
   __syncthreads();
-  /* half-sweep J of the launch is half-sweep J % 2nc of its iteration J / 2nc,
+  /* half-sweep j of the launch is half-sweep j % 2nc of its iteration j / 2nc,
    * whose demons sit one walk step further per iteration */
-  const unsigned per_it = 2u * (unsigned)g.nc, J = job[1];
-  const unsigned jj = J % per_it;
-  const int kwalk = (int)((job[6] + J / per_it) % (unsigned)g.Lh);
   if (pf > 0) {
     /* the tile's demon words are independent of the half-sweep before it:
      * on their way into L2 while the lead thread waits for the dependencies
      * (at most pf planes: the z loop's own prefetch takes over from there) */
-    if (!micsa_frozen(g, (int)job[0]))
-      prefetch_tile_demons<VW>(g, (int)(jj & 1u), (int)(jj >> 1), job[0], job[5], job[4],
-                               job[3], job[2] * (unsigned)zc, pf < zc ? pf : zc, kwalk, d0, d1);
-    if (lead) dep_wait(g, ctl, cst, job);
+    if (!LIN && job[J_RUN])
+      prefetch_tile_demons<VW>(g, (int)(job[J_HALF] & 1u), (int)(job[J_HALF] >> 1), job[J_S],
+                               job[J_GRP], job[J_Y], job[J_X], job[J_SLAB] * (unsigned)zc,
+                               pf < zc ? pf : zc, (int)(job[J_WALK] % (unsigned)g.Lh), d0, d1);
+    if (lin < 32u) flow_wait_lanes(c, need, ok);
     __syncthreads();
   }
-  {
-    const unsigned s = job[0];
-    if (!micsa_frozen(g, (int)s)) {
-      micsa_tma none;
-      sweep_block<VW, true, WIDE, false, true, 2, false, XS, UNR>(
-          g, (int)(jj & 1u), (int)(jj >> 1), s, job[5], job[4], job[3], job[2] * (unsigned)zc,
-          zc, pd, kwalk, spin, d0, d1, jb, nullptr, none);
+  if (job[J_RUN]) {
+    micsa_tma none;
+    unsigned y = job[J_Y], x = job[J_X];
+    if (LIN) {
+      const unsigned u = y * blockDim.x + threadIdx.x;
+      y = f.pairs(u);
+      x = u - y * f.pairs.d;
     }
+    sweep_block<VW, true, WIDE, false, true, S, LIN, XS, UNR>(
+        g, (int)(job[J_HALF] & 1u), (int)(job[J_HALF] >> 1), job[J_S], job[J_GRP], y, x,
+        job[J_SLAB] * (unsigned)zc, zc, pd, (int)(job[J_WALK] % (unsigned)g.Lh), spin, d0, d1, jb, nullptr, none);
   }
-  __syncthreads();
-  if (lead) {
-    __threadfence();
-    atomicAdd(ctl + 4 + job[0] * cst[C_NSLAB] + job[2], 1u);
-    __threadfence();
-    job[7] = atomicAdd(ctl + 1, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (job[7]) { /* every other block has finished: reset for the next launch */
-    const unsigned tid = threadIdx.y * blockDim.x + threadIdx.x, nt = blockDim.x * blockDim.y;
-    const unsigned n = (unsigned)g.ns * cst[C_NSLAB];
-    for (unsigned k = tid; k < n; k += nt) ctl[4 + k] = 0;
-    if (lead) {
-      ctl[0] = 0;
-      ctl[1] = 0;
+  __syncwarp();
+  if ((lin & 31u) == 0) {
+    const unsigned warps = (blockDim.x * blockDim.y + 31u) / 32u;
+    if (add_acq_rel_cta(&done, 1u) == warps - 1u) {
+      red_release_gpu(ctl + 4 + job[J_S] * f.nslab.d + job[J_SLAB], 1u);
     }
   }
 }
@@ -2157,14 +2242,35 @@ static cudaError_t sweep_flow_k(const micsa_geo &g, int smaj, int ytiles, int G,
     return launch_sweep(g, k_sweep_pdep<VW, WIDE, MINB>, dim3((unsigned)nb), block, 0, st, g,
                         ytiles, G, zc, g.pd, smaj, (unsigned)tiles, spin, d0, d1, jb, walk, ctl);
   }
-  if (g.half) /* half-height tiles: the same registers per thread, twice the blocks per SM */
-    return launch_sweep(g, k_sweep_dep<VW, WIDE, 2 * MINB, TPB / 2>, dim3((unsigned)tiles), block,
-                        0, st, g, ytiles, G, zc, g.pd, smaj, g.pf, spin, d0, d1, jb, walk, ctl);
-  if (g.xs) /* the x halo by warp shuffle */
-    return launch_sweep(g, k_sweep_dep<VW, WIDE, MINB, TPB, true>, dim3((unsigned)tiles), block,
-                        0, st, g, ytiles, G, zc, g.pd, smaj, g.pf, spin, d0, d1, jb, walk, ctl);
-  return launch_sweep(g, k_sweep_dep<VW, WIDE, MINB>, dim3((unsigned)tiles), block, 0, st, g,
-                      ytiles, G, zc, g.pd, smaj, g.pf, spin, d0, d1, jb, walk, ctl);
+  const bool lin = g.tw == 2;
+  const unsigned gx = lin ? 1u : (unsigned)g.Lh / 2u / block.x, nslab = (unsigned)(g.L / zc);
+  const unsigned T = gx * (unsigned)ytiles * (unsigned)G, half = nslab * T;
+  const unsigned halves = (unsigned)(g.fit > 1 ? g.fit : 1) * 2u * (unsigned)g.nc;
+  const micsa_flow_plan f = {micsa_udiv(smaj ? halves * half : (unsigned)g.ns * half), micsa_udiv(half),
+                             micsa_udiv(T), micsa_udiv(gx), micsa_udiv((unsigned)ytiles),
+                             micsa_udiv(nslab), micsa_udiv(2u * (unsigned)g.nc),
+                             micsa_udiv((unsigned)g.Lh / (g.quad ? 4u : 2u)), smaj};
+  const dim3 grid((unsigned)tiles);
+  cudaError_t e = cudaErrorInvalidValue;
+  if (lin && g.quad) {
+    if constexpr (VW == 1 && WIDE)
+      e = launch_sweep(g, k_sweep_dep<VW, WIDE, MINB, TPB, false, true, 4>, grid, block, 0, st, g, f,
+                       zc, g.pd, 0, spin, d0, d1, jb, walk, ctl);
+  } else if (lin)
+    e = launch_sweep(g, k_sweep_dep<VW, WIDE, MINB, TPB, false, true>, grid, block, 0, st, g, f, zc,
+                     g.pd, 0, spin, d0, d1, jb, walk, ctl);
+  else if (g.half) /* half-height tiles: the same registers per thread, twice the blocks per SM */
+    e = launch_sweep(g, k_sweep_dep<VW, WIDE, 2 * MINB, TPB / 2>, grid, block, 0, st, g, f, zc, g.pd,
+                     g.pf, spin, d0, d1, jb, walk, ctl);
+  else if (g.xs) /* the x halo by warp shuffle */
+    e = launch_sweep(g, k_sweep_dep<VW, WIDE, MINB, TPB, true>, grid, block, 0, st, g, f, zc, g.pd,
+                     g.pf, spin, d0, d1, jb, walk, ctl);
+  else
+    e = launch_sweep(g, k_sweep_dep<VW, WIDE, MINB>, grid, block, 0, st, g, f, zc, g.pd, g.pf, spin,
+                     d0, d1, jb, walk, ctl);
+  if (e != cudaSuccess) return e;
+  /* the counters are zero again for the next launch */
+  return cudaMemsetAsync(ctl, 0, sizeof(unsigned) * (4 + (size_t)g.ns * nslab), st);
 }
 
 template <int VW>
@@ -2175,11 +2281,14 @@ static cudaError_t sweep_flow_vw(const micsa_geo &g, int smaj, uint32_t *spin, u
   int tx, ty;
   sweep_tile(g.L, g.tw, &tx, &ty);
   if (g.half && !g.pers) ty = ty / 2 > 0 ? ty / 2 : 1; /* blocks of tx x ty/2 threads */
-  const int ytiles = (g.L + ty - 1) / ty;
+  const bool lin = g.tw == 2; /* consecutive units of two sites (four: g.quad) */
+  if (lin) { tx = TPB; ty = 1; }
+  const int units = g.L * g.Lh / (g.quad ? 4 : 2);
+  const int ytiles = lin ? (units + TPB - 1) / TPB : (g.L + ty - 1) / ty;
   const int zc = g.zc > 0 ? g.zc : 4;
   if (g.L % zc) return cudaErrorInvalidValue;
   const int64_t tiles = (int64_t)(g.fit > 1 ? g.fit : 1) * g.ns * 2 * g.nc * (g.L / zc) *
-                        (g.Lh / 2 / tx) * ytiles * G;
+                        (lin ? 1 : g.Lh / 2 / tx) * ytiles * G;
   if (tiles >= (1LL << 31)) return cudaErrorInvalidValue; /* 32-bit tickets */
   const dim3 block(tx, ty);
   constexpr int B0 = VW == 4 ? 2 : 3, B1 = VW == 4 ? 2 : 4;
@@ -2406,6 +2515,13 @@ int micsa_sweep_wide_differs(int L, int sites) {
 int micsa_sweep_zc_candidates(int L, int *out, int max) {
   int n = 0;
   for (int zc = 1; zc <= 64 && zc <= L && n < max; zc <<= 1)
+    if (L % zc == 0) out[n++] = zc;
+  return n;
+}
+
+int micsa_flow_zc_candidates(int L, int *out, int max) {
+  int n = 0;
+  for (int zc = 2; zc <= 16 && zc <= L && n < max; zc++)
     if (L % zc == 0) out[n++] = zc;
   return n;
 }

@@ -34,9 +34,11 @@ struct micsa_geo {
   int async;  /* 1: the sweep double-buffers each step's operands with cp.async (W = 2) */
   int pipe;   /* 1: the sweep loads each z step's operands into registers one step ahead */
   int pdl;    /* 1: sweeps launched with programmatic dependent launch */
-  int tw;     /* 1: sweep blocks span whole rows along x (when that differs) */
+  int tw;     /* 1: sweep blocks span whole rows along x (when that differs);
+               * 2: blocks of consecutive (row, x/2) units (dataflow sweep) */
   int flow;   /* 1: an iteration's half-sweeps run as one dataflow launch */
-  int quad;   /* 1: four one-word sites per sweep thread (W = 1, direct loads) */
+  int quad;   /* 1: four one-word sites per sweep thread (W = 1, direct loads or
+               * the dataflow sweep with tw = 2) */
   int pf;     /* dataflow sweep: demon planes of its tile requested into L2 before its
                  dependency wait (0 = none) */
   int fit;    /* dataflow sweep: iterations carried by one launch (>= 1) */
@@ -78,6 +80,8 @@ int micsa_sweep_wide_differs(int L, int sites = 2);
 
 /* slab depths the sweep can use for this L (divisors of L, ascending) */
 int micsa_sweep_zc_candidates(int L, int *out, int max);
+/* ... and the dataflow sweep (all divisors of L from 2 to 16) */
+int micsa_flow_zc_candidates(int L, int *out, int max);
 
 /* flag = 1 half-sweep of colour p on demon plane ic, all samples; with
  * g.tma and tm->ok the demon tiles are staged by TMA */

@@ -19,6 +19,7 @@
 
 #include "micsa.h"
 #include "micsa_host.h"
+#include "micsa_internal.h"
 
 #define MAXNSAMPLES_REF 2 /* header.h:20, sizes the reference's seed fan-out */
 
@@ -458,7 +459,7 @@ int micsa_run_batch(int device, const micsa_job *jobs, int njobs, int32_t *e_spi
                            maxH, maxnr, J, even, odd, prc, xo, e_spin, e_demon, MICSA_OK, {0}};
       const micsa_job *j0 = &jobs[idx[gstart[g]]];
       micsa_config cfg = {device, j0->L, j0->nr, grs[g].n, j0->nc};
-      if ((grs[g].rc = micsa_create(&cfg, &grs[g].ctx)))
+      if ((grs[g].rc = ng > 1 ? micsa_create_shared(&cfg, &grs[g].ctx) : micsa_create(&cfg, &grs[g].ctx)))
         snprintf(grs[g].err, sizeof grs[g].err, "micsa_create L=%d nr=%d n=%d failed (%d)", j0->L,
                  j0->nr, grs[g].n, grs[g].rc);
     }

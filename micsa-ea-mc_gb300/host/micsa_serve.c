@@ -29,6 +29,7 @@
 
 #include "micsa.h"
 #include "micsa_host.h"
+#include "micsa_internal.h"
 
 #define MAXNSAMPLES_REF 2 /* header.h:20, sizes the reference's seed fan-out */
 
@@ -461,7 +462,7 @@ int micsa_server_create(const micsa_server_config *cfg, micsa_server **out, char
     }
     /* contexts are created (and tuned) here, before any request: a warm server */
     micsa_config c = {cfg->device, pl->L, pl->nr, S, pl->nc};
-    if ((rc = micsa_create(&c, &pl->ctx))) {
+    if ((rc = micsa_create_shared(&c, &pl->ctx))) {
       if (err && errlen) snprintf(err, errlen, "micsa_create L=%d nr=%d S=%d failed", pl->L, pl->nr, S);
       break;
     }
