@@ -290,6 +290,52 @@ struct quads {
 template <int VW, bool WIDE, int S> struct sites_io { using type = pairs<VW, WIDE>; };
 template <> struct sites_io<1, true, 4> { using type = quads; };
 
+/* The bond masks of a thread's S sites from their coupling bytes (site k's
+ * byte in bits 8k .. 8k+7, 6 bits each).  A byte permute that replicates the
+ * sign bit of one byte makes a mask of it in one instruction, so each bond
+ * bit is moved to the top of its byte first, for all sites at once; with two
+ * sites one multiplication does that for two bonds (the shifted copies do
+ * not overlap), off the ALU pipe: 16 ALU and multiply operations for the 12
+ * masks where single bit extracts take 24.  With the x neighbours below and
+ * W a constant where it is one: us per iteration of the dataflow sweep 344 ->
+ * 320 (L=160, 2 samples x 64 replicas), 96 -> 87 (L=64, 8 x 64); of the
+ * half-sweep launches 159 -> 155 (L=128, 2 x 64). */
+__device__ __forceinline__ uint32_t byte_sign(uint32_t x, int byte) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(x), "r"(0x8888u + 0x1111u * (unsigned)byte));
+  return r;
+}
+template <int S> struct micsa_bonds {
+  uint32_t c, b, n, s, u, d;
+  __device__ __forceinline__ micsa_bonds(uint32_t jb, uint32_t rowoff) {
+    const uint32_t e = jb << 7, o = jb << 4;
+    c = rowoff ? o : e;
+    b = rowoff ? e : o;
+    n = jb << 6; u = jb << 5; s = jb << 3; d = jb << 2;
+  }
+  __device__ __forceinline__ uint32_t column(int k) const { return byte_sign(c, k); }
+  __device__ __forceinline__ uint32_t beside(int k) const { return byte_sign(b, k); }
+  __device__ __forceinline__ uint32_t north(int k) const { return byte_sign(n, k); }
+  __device__ __forceinline__ uint32_t up(int k) const { return byte_sign(u, k); }
+  __device__ __forceinline__ uint32_t south(int k) const { return byte_sign(s, k); }
+  __device__ __forceinline__ uint32_t down(int k) const { return byte_sign(d, k); }
+};
+template <> struct micsa_bonds<2> {
+  uint32_t x, un, ds; /* bytes 0, 1 and bytes 2, 3: one bond each, of both sites */
+  __device__ __forceinline__ micsa_bonds(uint32_t jb, uint32_t rowoff) {
+    const uint32_t oe = jb * ((1u << 4) | (1u << 23)); /* -x, +x */
+    x = __funnelshift_l(oe, oe, 16u * (rowoff ^ 1u));
+    un = jb * ((1u << 5) | (1u << 22)); /* +z, +y */
+    ds = jb * ((1u << 2) | (1u << 19)); /* -z, -y */
+  }
+  __device__ __forceinline__ uint32_t column(int k) const { return byte_sign(x, k); }
+  __device__ __forceinline__ uint32_t beside(int k) const { return byte_sign(x, k + 2); }
+  __device__ __forceinline__ uint32_t up(int k) const { return byte_sign(un, k); }
+  __device__ __forceinline__ uint32_t north(int k) const { return byte_sign(un, k + 2); }
+  __device__ __forceinline__ uint32_t down(int k) const { return byte_sign(ds, k); }
+  __device__ __forceinline__ uint32_t south(int k) const { return byte_sign(ds, k + 2); }
+};
+
 __device__ __forceinline__ uint32_t ld_u32_keep(const uint8_t *a, uint64_t pol) {
   uint32_t v;
   asm("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(v) : "l"(a), "l"(pol));
@@ -341,7 +387,7 @@ __device__ __forceinline__ void sweep_block(
   static_assert(!XS || (S == 2 && !LIN && !TMA), "x halo by shuffle: pairs, block-shaped tiles");
   constexpr int N = S * VW; /* words per thread and plane */
   using PR = typename sites_io<VW, WIDE, S>::type;
-  const uint32_t L = g.L, Lh = g.Lh, W = g.W;
+  const uint32_t L = g.L, Lh = g.Lh, W = WIDE ? (uint32_t)VW : (uint32_t)g.W;
   const uint32_t y = LIN ? tile : tile * blockDim.y + threadIdx.y;
   /* XS: the lanes of this warp that stay (rows inside the lattice) */
   unsigned xs_mask = 0;
@@ -548,33 +594,25 @@ __device__ __forceinline__ void sweep_block(
       PR::ld_na(rb + 2 * P * W, W, a2, strm);
     }
     /* x-neighbours: the thread's site k (x/2 = xa + k) of colour p sees, in
-     * the other colour, +x at x/2 + rowoff and -x at x/2 + rowoff - 1: words
-     * of v0, or ext past either end */
+     * the other colour, +x at x/2 + rowoff and -x at x/2 + rowoff - 1: its own
+     * column's word v0[k] (the +x neighbour, or with rowoff the -x one) and
+     * the word beside it, k - 1 (with rowoff k + 1), or ext past either end.
+     * The six counts are added without regard to direction, so it is the
+     * coupling bits that are chosen by rowoff, once per thread and plane, and
+     * one word per site word, not both neighbours of each. */
+    const micsa_bonds<S> bonds(jbs, rowoff);
 #pragma unroll
     for (int site = 0; site < S; site++) {
-      const uint32_t jb6 = (jbs >> (8 * site)) & 0xffu;
-      const uint32_t mE = jmask(jb6, 0), mN = jmask(jb6, 1), mU = jmask(jb6, 2);
-      const uint32_t mO = jmask(jb6, 3), mS = jmask(jb6, 4), mD = jmask(jb6, 5);
+      const uint32_t mC = bonds.column(site), mN = bonds.north(site), mU = bonds.up(site);
+      const uint32_t mB = bonds.beside(site), mS = bonds.south(site), mD = bonds.down(site);
 #pragma unroll
       for (int w = 0; w < VW; w++) {
         const int o = site * VW + w;
-        /* site k: +x = rowoff ? (k+1 < S ? v0[k+1] : ext) : v0[k],
-         *         -x = rowoff ? v0[k] : (k > 0 ? v0[k-1] : ext) */
-        uint32_t nE, nO;
-        if constexpr (S == 2) { /* A = site 0, B = site 1 */
-          const uint32_t cA = v0[w], cB = v0[VW + w], ex = ext[w];
-          nE = site == 0 ? (rowoff ? cB : cA) : (rowoff ? ex : cB);
-          nO = site == 0 ? (rowoff ? cA : ex) : (rowoff ? cB : cA);
-        } else {
-          const uint32_t ck = v0[o], ex = ext[w];
-          const uint32_t cn = site + 1 < S ? v0[(site + 1 < S ? site + 1 : 0) * VW + w] : ex;
-          const uint32_t cp = site > 0 ? v0[(site > 0 ? site - 1 : 0) * VW + w] : ex;
-          nE = rowoff ? cn : ck;
-          nO = rowoff ? ck : cp;
-        }
-        const uint32_t sw = own[o];
-        const uint32_t f0 = xor3(sw, nE, mE), f1 = xor3(sw, vn[o], mN), f2 = xor3(sw, up[o], mU);
-        const uint32_t f3 = xor3(sw, nO, mO), f4 = xor3(sw, vs[o], mS), f5 = xor3(sw, vm[o], mD);
+        const uint32_t next = site + 1 < S ? v0[(site + 1 < S ? site + 1 : 0) * VW + w] : ext[w];
+        const uint32_t prev = site > 0 ? v0[(site > 0 ? site - 1 : 0) * VW + w] : ext[w];
+        const uint32_t sw = own[o], nB = rowoff ? next : prev;
+        const uint32_t f0 = xor3(sw, v0[o], mC), f1 = xor3(sw, vn[o], mN), f2 = xor3(sw, up[o], mU);
+        const uint32_t f3 = xor3(sw, nB, mB), f4 = xor3(sw, vs[o], mS), f5 = xor3(sw, vm[o], mD);
         const uint32_t j1 = xor3(f0, f1, f2), j2 = maj3(f0, f1, f2);
         const uint32_t j3 = xor3(f3, f4, f5), j4 = maj3(f3, f4, f5);
         uint32_t flip;
