@@ -54,6 +54,7 @@ struct micsa_ctx {
   int64_t launches = 0;
   int resident = 0;        /* small lattice: iterations run in shared memory, by clusters of
                               this many blocks per sample and replica word (0: not) */
+  int resident_once = 0;    /* of these clusters the GPU runs at once (0: not asked) */
   int64_t resident_min = 1; /* calls of fewer iterations run half-sweep by half-sweep */
   int split = 0;           /* k > 0: half-sweep launches per group of k samples, group-major
                               (a smaller L2 working set); 0: all samples per launch */
@@ -939,7 +940,9 @@ int create_ctx(const micsa_config *cfg, bool shared, micsa_ctx **out) {
     if (!(er && !strcmp(er, "0")) && (cfg->L <= 16 || !getenv("MICSA_SWEEP_ZC")))
       MICSA_CK_CREATE(micsa_resident_shape(cfg->L, cfg->nc, g.W, cfg->nsamples, optin,
                                            ec ? atoi(ec) : 0, &ctx->resident,
-                                           &ctx->resident_min));
+                                           &ctx->resident_once, &ctx->resident_min));
+    /* beside other contexts' kernels a last wave leaves them its SMs */
+    if (shared) ctx->resident_once = 0;
   }
   MICSA_CK_CREATE(micsa_make_tma(ctx->g, ctx->dem0, ctx->dem1, &ctx->tma));
   if ((rc = autotune(ctx)) != MICSA_OK) {
@@ -1423,7 +1426,7 @@ int micsa_iterate(micsa_ctx *ctx, int64_t n) {
   if (!ctx->graph_exec && !resident && n >= unit &&
       (rc = capture_iterations(ctx, unit, &ctx->graph, &ctx->graph_exec, &ctx->graph_launches)))
     return rc;
-  const int left = unit > 1 ? (int)(n % unit) : 0;
+  const int left = unit > 1 && !resident ? (int)(n % unit) : 0;
   if (left) {
     if (ctx->rem_exec.size() < (size_t)unit) {
       ctx->rem_graph.resize((size_t)unit, nullptr);
@@ -1439,9 +1442,8 @@ int micsa_iterate(micsa_ctx *ctx, int64_t n) {
     /* small lattices: whole iterations in shared memory, up to 1024 per launch */
     for (int64_t done = 0; done < n;) {
       const int m = (int)(n - done < 1024 ? n - done : 1024);
-      MICSA_CK(micsa_launch_resident(ctx->g, ctx->resident, m, ctx->spin, ctx->dem0, ctx->dem1, ctx->jb,
-                                     ctx->walk, ctx->stream));
-      ctx->launches += 2;
+      MICSA_CK(micsa_launch_resident(ctx->g, ctx->resident, ctx->resident_once, m, ctx->spin, ctx->dem0,
+                                     ctx->dem1, ctx->jb, ctx->walk, ctx->stream, &ctx->launches));
       done += m;
     }
     return MICSA_OK;

@@ -95,8 +95,15 @@ template <int L, int C, int PPT> struct rcfg {
   }
 };
 
-/* n iterations of sample blockIdx.z, replica word blockIdx.y, by one cluster
- * along blockIdx.x.
+/* A launch's share of a call of `total` iterations of `units` (sample,
+ * replica word) pairs in `rounds` rounds: cluster i takes place first + i of
+ * the sequence (round 0 of every unit, round 1 of every unit, ...). */
+struct slice {
+  int total, rounds, units, first;
+};
+
+/* n iterations of one sample and replica word by one cluster along
+ * blockIdx.x: all of the call's, or one round's (see slice).
  *
  * Shared memory: sp[2][HZ][PL] spins (with C > 1 a halo plane below and
  * above the slab), then the demon planes [(p, ic)][Zc][PL][D0, D1].  A
@@ -139,11 +146,12 @@ template <int L, int C, int PPT> struct rcfg {
  * D0 and D1 apart 0.87, the pushes spread over three half-sweeps 0.86; one
  * pair per thread (64 registers) 1.16.  Measured against the half-sweep
  * launches: L=16, one sample x 64 replicas 11.3 -> 3.2 us per iteration;
- * L=24, 2 x 32, nc=5 23.1 -> 5.5; L=32, 24 x 64 65 -> 41 (15 clusters of
- * 221 KB per block fit the GPU at once: four waves). */
+ * L=24, 2 x 32, nc=5 23.1 -> 5.5; L=32, 24 x 64 65 -> 33 (15 clusters of
+ * 221 KB per block fit the GPU at once; 39 in four waves, see
+ * resident_rounds). */
 template <int L, int C, int PPT>
 __global__ void __launch_bounds__((rcfg<L, C, PPT>::T), 1)
-k_resident(const micsa_geo g, const int n, uint32_t *__restrict__ spin,
+k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
            uint32_t *__restrict__ d0, uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb,
            const int *__restrict__ walk) {
   using K = rcfg<L, C, PPT>;
@@ -154,14 +162,18 @@ k_resident(const micsa_geo g, const int n, uint32_t *__restrict__ spin,
   constexpr uint32_t PB = PL * 4; /* bytes of a spin plane */
   extern __shared__ uint4 smem_raw[];
   __shared__ uint64_t bars[6]; /* halo of colour 0, 1; demons of (ic 2, p), (ic 5, p) */
-  const int rank = CL ? (int)blockIdx.x : 0, w = blockIdx.y, s = blockIdx.z, W = g.W, nc = g.nc;
+  const int rank = CL ? (int)blockIdx.x : 0, W = g.W, nc = g.nc;
+  const int place = sl.first + (int)(blockIdx.z * gridDim.y + blockIdx.y), round = place / sl.units, unit = place - round * sl.units;
+  const int w = unit % W, s = unit / W;
+  const int share = sl.total / sl.rounds, more = sl.total % sl.rounds;
+  const int n = share + (round < more), done = round * share + (round < more ? round : more);
   if (micsa_frozen(g, s)) return; /* the whole cluster */
   char *const sm = (char *)smem_raw;
   uint32_t *const sp = (uint32_t *)smem_raw;
   uint2 *const sd = (uint2 *)(sp + 2 * HZ * PL); /* [2*nc][Zc][PL] (D0, D1) */
   const int tid = threadIdx.x, z0 = rank * Zc;
   const size_t sbase = (size_t)s * 2 * P, dbase = (size_t)s * 2 * nc * P;
-  const int k0 = walk[s];
+  const int k0 = (walk[s] + done) % Lh;
 
   /* spins of the slab (and its halos); demons, the planes that the walk
    * moves along z already in the frame of their sites: a pair of sites per
@@ -443,7 +455,7 @@ k_resident(const micsa_geo g, const int n, uint32_t *__restrict__ spin,
 }
 
 /* ------------------------------------------------------------- launches */
-using kern_t = void (*)(micsa_geo, int, uint32_t *, uint32_t *, uint32_t *, const uint8_t *,
+using kern_t = void (*)(micsa_geo, slice, uint32_t *, uint32_t *, uint32_t *, const uint8_t *,
                         const int *);
 struct variant {
   int L, C, T;
@@ -496,8 +508,9 @@ cudaError_t config(const variant &v, int nc, int W, int ns, cudaStream_t st,
  * (48 against 62; n = 1: 38 against 31), four waves (L=32 x 24 samples) from
  * n = 5 (n = 4: 245 against 243 us, n = 8: 399 against 486). */
 cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pin, int *cluster,
-                                 int64_t *min_n) {
+                                 int *at_once, int64_t *min_n) {
   *cluster = 0;
+  *at_once = 0;
   *min_n = 1;
   int n;
   const variant *v = variants(&n);
@@ -513,24 +526,55 @@ cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pi
     const int64_t waves = ((int64_t)W * ns + fit - 1) / fit;
     if (*cluster == 0 || waves == 1) {
       *cluster = v[i].C;
+      *at_once = pin > 0 ? 0 : fit;
       *min_n = pin > 0 ? 1 : waves + (waves > 1 || L > 24);
     }
   }
   return cudaSuccess;
 }
 
-cudaError_t micsa_launch_resident(const micsa_geo &g, int cluster, int n, uint32_t *spin,
+/* Rounds for a call of n iterations.  U clusters of which M run at once take
+ * ceil(U / M) waves, the last one mostly idle when U is a little more than a
+ * multiple of M; in R rounds of n / R iterations, laid end to end and cut
+ * into launches of M, only the last of ceil(R*U / M) launches is.  A wave
+ * costs its iterations and about four more (its share of copying the state
+ * in and out, the launch).  us per iteration at 256 iterations: L=32, 24
+ * samples x 64 replicas (U = 48, M = 15; 16 launches of 51 iterations for 4
+ * waves of 256) 38.9 -> 32.8; L=32, 10 x 64 19.4 -> 13.5; L=24, 24 x 64 17.9 ->
+ * 12.2; L=16, 100 x 64 14.4 -> 9.8.  Launches side by side on two streams
+ * gained another 1% and were left out. */
+static int resident_rounds(int64_t U, int64_t M, int n) {
+  if (M < 1 || U <= M) return 1;
+  int best = 1;
+  double cost = 0.97 * (double)((U + M - 1) / M) * (n + 4); /* 3% less, or not worth it */
+  for (int R = 2; R <= 8 && R <= n; R++) {
+    const double c = (double)((R * U + M - 1) / M) * ((double)n / R + 4);
+    if (c < cost) cost = c, best = R;
+  }
+  return best;
+}
+
+cudaError_t micsa_launch_resident(const micsa_geo &g, int cluster, int at_once, int n, uint32_t *spin,
                                   uint32_t *d0, uint32_t *d1, const uint8_t *jb, int *walk,
-                                  cudaStream_t st) {
+                                  cudaStream_t st, int64_t *launches) {
   int nv;
   const variant *v = variants(&nv);
+  const int U = g.W * g.ns, R = resident_rounds(U, at_once, n), M = R > 1 ? at_once : U;
   for (int i = 0; i < nv; i++) {
     if (v[i].L != g.L || v[i].C != cluster) continue;
     cudaLaunchAttribute at;
     cudaLaunchConfig_t c;
-    cudaError_t e = config(v[i], g.nc, g.W, g.ns, st, &at, &c);
-    if (e == cudaSuccess) e = cudaLaunchKernelEx(&c, v[i].k, g, n, spin, d0, d1, jb, (const int *)walk);
-    return e != cudaSuccess ? e : micsa_launch_walk_add(g, walk, n, st);
+    cudaError_t e = R > 1 ? config(v[i], g.nc, M, 1, st, &at, &c) : config(v[i], g.nc, g.W, g.ns, st, &at, &c);
+    for (int first = 0; first < R * U && e == cudaSuccess; first += M) {
+      /* exactly the places that are left: a test for them in the kernel cost
+       * its half-sweeps 8% (L=32) */
+      if (R > 1) c.gridDim.y = (unsigned)(R * U - first < M ? R * U - first : M);
+      e = cudaLaunchKernelEx(&c, v[i].k, g, slice{n, R, U, first}, spin, d0, d1, jb, (const int *)walk);
+      ++*launches;
+    }
+    if (e != cudaSuccess) return e;
+    ++*launches;
+    return micsa_launch_walk_add(g, walk, n, st);
   }
   return cudaErrorInvalidValue;
 }

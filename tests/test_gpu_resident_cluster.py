@@ -82,3 +82,28 @@ def test_frozen_samples_and_refresh_between_cluster_launches():
     _same(a, b, ns, "mixed")
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("L,nr,nc,ns,n", [
+    (32, 64, 6, 10, 20),   # 20 clusters where 15 run at once: two launches share units
+    (32, 96, 6, 11, 40),   # 33 clusters; rounds of unequal length
+    (32, 32, 6, 17, 33),   # more than one walk period
+    (24, 64, 6, 20, 40)])  # more clusters than run at once with the smaller cluster too
+def test_rounds_equal_half_sweep_kernels(L, nr, nc, ns, n):
+    """Calls cut into rounds over several launches, each unit's walk going on
+    from its round before, and the calls after them."""
+    rng = np.random.default_rng(L + nr + ns)
+    st = random_state(rng, L, nr, nc, ns)
+    a = _ctx(L, nr, ns, nc, {}, st)
+    b = _ctx(L, nr, ns, nc, {"MICSA_RESIDENT": "0"}, st)
+    for k in (n, 1, n + 3):
+        for c in (a, b):
+            c.iterate(k)
+        _same(a, b, ns, k)
+    if L == 32: # the largest one: 15 clusters at once
+        l0 = a.kernel_launches()
+        a.iterate(n)
+        assert a.kernel_launches() - l0 > 2  # several rounds
+    a.synchronize()
+    a.close()
+    b.close()
