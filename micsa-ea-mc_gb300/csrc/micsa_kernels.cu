@@ -139,6 +139,9 @@ __device__ __forceinline__ int64_t demon_slot(const micsa_geo &g, int p, int ic,
 /* Programmatic dependent launch: let the next grid in the stream be
  * scheduled now, then wait until the previous grid has completed and its
  * memory operations are visible (a no-op for a plain launch). */
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void grid_dependency_sync() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -668,6 +671,7 @@ k_sweep(const micsa_geo g, const int p, const int ic, const int ytiles, const in
         uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb,
         const int *__restrict__ walk, const uint32_t *__restrict__ rnd,
         const __grid_constant__ micsa_tma tm) {
+  if (!MICSA) grid_launch_dependents(); /* the next colour's bits are drawn beside this sweep */
   grid_dependency_sync();
   const uint32_t by = blockIdx.y;
   const uint32_t tile = by % ytiles, sg = by / ytiles; /* block-uniform */
@@ -1648,6 +1652,7 @@ k_gen_rnd(const __grid_constant__ micsa_geo g, const int p, const __grid_constan
   __shared__ uint4 s_te[Source::STAGE];
   __shared__ uint32_t s_key[Source::STAGE];
   __shared__ uint8_t s_late[TPB / 32][2 * 32 * 4]; /* bytes found by bisection, [call][lane][byte] */
+  grid_launch_dependents();
   const uint4 *bins = reinterpret_cast<const uint4 *>(lut + 4096);
   for (int t = threadIdx.x; t < 512; t += TPB) s_bin4[t] = __ldg(bins + t);
   const uint2 *s_bin = reinterpret_cast<const uint2 *>(s_bin4);
@@ -1661,10 +1666,12 @@ k_gen_rnd(const __grid_constant__ micsa_geo g, const int p, const __grid_constan
   __syncthreads();
   if (tid >= (uint32_t)g.H * (uint32_t)g.nr) return; /* warp-uniform: H*nr is a multiple of 32 */
   const uint4 t4 = from.counter(r, s_te);
-  uint32_t c[4] = {t4.x, t4.y, t4.z + tid, t4.w};
+  /* the words blockIdx.y, + gridDim.y, ... of the three: two calls each */
+  uint32_t c[4] = {t4.x + 2u * blockIdx.y, t4.y, t4.z + tid, t4.w};
   const uint32_t key1 = from.key(r, s_key);
   const site_xyz site = ref_site(g, p, h, lane);
-  uint32_t *out = rnd + (((int64_t)site.z * g.L + site.y) * g.Lh + (site.x >> 1)) * g.W + (r >> 5);
+  uint32_t *out = rnd + (((int64_t)site.z * g.L + site.y) * g.Lh + (site.x >> 1)) * g.W + (r >> 5) +
+                  (int64_t)blockIdx.y * g.P * g.W;
   int waiting = 0; /* draws in the warp's queue */
   auto bisect32 = [&](int at) { /* queue entries at .. at+31, as far as there are any */
     __syncwarp();
@@ -1677,7 +1684,7 @@ k_gen_rnd(const __grid_constant__ micsa_geo g, const int p, const __grid_constan
     __syncwarp();
   };
 #pragma unroll 1
-  for (int word = 0; word < 3; word++) {
+  for (int word = (int)blockIdx.y; word < 3; word += (int)gridDim.y) {
     uint32_t rot[2], wd[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -1711,6 +1718,7 @@ k_gen_rnd(const __grid_constant__ micsa_geo g, const int p, const __grid_constan
       late[q * 32 + lane] = 0;
       wd[q] = __funnelshift_l(bb, bb, rot[q]);
     }
+    if (word == (int)blockIdx.y) grid_dependency_sync(); /* the last sweep has read the old bits */
     /* 64-bit word = (wd[0] << 32) | wd[1]; bit b = block b; the block of bit
      * lane + 32 is two blocks up along z */
     out[0] = warp_transpose32(wd[1], lane);
@@ -2445,11 +2453,30 @@ void micsa_lut_bins(const void *lut, uint32_t *bins) {
   }
 }
 
+/* The three words of a site go to blocks of their own where all the blocks of
+ * one each would not give every SM one (a warp then runs one dependent chain
+ * of Philox calls, not three: L=32, 64 replicas 8.4 -> 5.4 us; L=64, 512
+ * blocks: 13.8 against 14.7, the table staged three times).  Launched as the
+ * sweeps are: the sweep of one colour lets the other colour's bits be drawn
+ * beside it, up to the first store (eight steps of L=64, 2 samples x 64
+ * replicas, read back: 428 -> 413 us; L=48, 1 x 128, four steps: 246 -> 209). */
+template <class Source>
+static cudaError_t launch_gen_rnd(const micsa_geo &g, int p, const Source &from, const uint8_t *lut,
+                                  uint32_t *rnd, cudaStream_t st) {
+  int dev = 0, nsm = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int blocks = blocks_for(g.H * g.nr, TPB);
+  e = launch_sweep(g, k_gen_rnd<Source>, dim3(blocks, blocks <= nsm ? 3 : 1), dim3(TPB), 0, st, g, p, from,
+                   lut, rnd);
+  return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 cudaError_t micsa_launch_gen_rnd(const micsa_geo &g, int p, const uint32_t *te,
                                  const uint32_t *keys, const uint8_t *lut, uint32_t *rnd,
                                  cudaStream_t st) {
-  k_gen_rnd<rnd_arrays><<<blocks_for(g.H * g.nr, TPB), TPB, 0, st>>>(g, p, rnd_arrays{te, keys}, lut, rnd);
-  return cudaGetLastError();
+  return launch_gen_rnd(g, p, rnd_arrays{te, keys}, lut, rnd, st);
 }
 
 cudaError_t micsa_launch_gen_rnd_values(const micsa_geo &g, int p, const uint32_t *te,
@@ -2458,8 +2485,7 @@ cudaError_t micsa_launch_gen_rnd_values(const micsa_geo &g, int p, const uint32_
   rnd_values v;
   memcpy(v.te, te, 16 * (size_t)g.nr);
   memcpy(v.keys, keys, 4 * (size_t)g.nr);
-  k_gen_rnd<rnd_values><<<blocks_for(g.H * g.nr, TPB), TPB, 0, st>>>(g, p, v, lut, rnd);
-  return cudaGetLastError();
+  return launch_gen_rnd(g, p, v, lut, rnd, st);
 }
 
 cudaError_t micsa_launch_walk_advance(const micsa_geo &g, int *walk, cudaStream_t st) {

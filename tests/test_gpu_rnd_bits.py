@@ -81,3 +81,25 @@ def test_metropolis_replica_counts(L, nr):
             oracle.metropolis_iteration(L, nr, J, e, o, te[:4 * nr].copy(), te[4 * nr:].copy(), keys, lut)
         ge, go = ctx.download_spins(0)
         assert np.array_equal(ge, e) and np.array_equal(go, o)
+
+
+@pytest.mark.parametrize("L,nr", [(8, 32), (40, 64), (48, 64), (16, 224)])  # 1, 125, 216 and 28 blocks
+def test_steps_back_to_back(L, nr):
+    """Steps queued one behind another, the bits of one colour drawn while the
+    sweep of the other still runs, by blocks of one word each (up to one block
+    per SM) or of all three."""
+    rng = np.random.default_rng(L * nr)
+    lut = runs.lut_bytes()[8:]
+    (J, e, o, *_r), = random_state(rng, L, nr, 1, 1)
+    keys = rng.integers(0, 1 << 32, size=nr, dtype=np.uint32)
+    te = rng.integers(0, 1 << 32, size=(6, 8 * nr), dtype=np.uint32)
+    with micsa.Context(L, nr, 1, 1) as ctx:
+        ctx.set_lut(lut)
+        ctx.upload_couplings(0, J)
+        ctx.upload_spins(0, e, o)
+        for t in te:
+            ctx.monte_carlo(0, t, keys)
+        for t in te:
+            oracle.metropolis_iteration(L, nr, J, e, o, t[:4 * nr].copy(), t[4 * nr:].copy(), keys, lut)
+        ge, go = ctx.download_spins(0)
+        assert np.array_equal(ge, e) and np.array_equal(go, o)
