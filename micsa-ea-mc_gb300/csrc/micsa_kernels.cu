@@ -683,6 +683,169 @@ k_sweep(const micsa_geo g, const int p, const int ic, const int ytiles, const in
                                               zc, pd, kwalk, spin, d0, d1, jb, rnd, tm);
 }
 
+template <int VW> struct step_ops {
+  uint32_t own[2 * VW], up[2 * VW], vn[2 * VW], vs[2 * VW], a0[2 * VW], a1[2 * VW], ext[VW];
+  uint32_t jb2;
+};
+
+/* One thread's columns of a half-sweep, as in sweep_block (pairs, direct
+ * loads), with loads of z step t+1 issued before the arithmetic and stores of
+ * step t: all of them (ALL), or its demon words and couplings only, which
+ * takes 9 instead of 27 registers: pairs of two-word sites fit 64 registers
+ * without spills.  The dataflow sweep's tiles use the latter (us per
+ * iteration, against all loads in their own step: L=160, 2 samples x 64
+ * replicas 320 -> 306; L=64, 8 x 64 87 -> 85; L=96, 8 x 32 169 -> 160; all
+ * loads early: 341 at L=160, 80 registers).  Issuing them early
+ * is safe: a thread's own spins and demon words are written only by that
+ * thread, the couplings are constant, and in a launch of one half-sweep (not
+ * FLOW) the other colour is read-only. */
+template <int VW, bool WIDE, bool FLOW, bool ALL>
+__device__ __forceinline__ void sweep_ahead_block(
+    const micsa_geo &g, const int p, const int ic, const uint32_t s, const uint32_t grp,
+    const uint32_t y, const uint32_t pair, const uint32_t z0, const int zc, const int pd,
+    const int kwalk, uint32_t *__restrict__ spin, uint32_t *__restrict__ d0,
+    uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb) {
+  constexpr int N = 2 * VW;
+  using PR = pairs<VW, WIDE>;
+  const uint32_t L = g.L, Lh = g.Lh, W = WIDE ? (uint32_t)VW : (uint32_t)g.W;
+  if (y >= L) return;
+  const uint32_t xa = 2 * pair;
+  const uint32_t plane = L * Lh;
+  const uint32_t row = y * Lh + xa;
+  const uint32_t rowN = (y + 1 == L) ? xa : row + Lh;
+  const uint32_t rowS = (y == 0) ? row + (L - 1) * Lh : row - Lh;
+  const uint32_t rowXp = (xa + 2 == Lh) ? row + 2 - Lh : row + 2;
+  const uint32_t rowXm = (xa == 0) ? row + Lh - 1 : row - 1;
+  const size_t P = (size_t)g.P;
+  uint32_t *mine = spin + (size_t)(s * 2 + p) * P * W + grp * VW;
+  const uint32_t *oth = spin + (size_t)(s * 2 + (p ^ 1)) * P * W + grp * VW;
+  const uint8_t *jbp = jb + (size_t)(s * 2 + p) * P;
+  const uint64_t keep = l2_keep(), strm = l2_stream();
+
+  uint32_t drowA = row, drowB = row + 1, zd = z0;
+  bool dpair = true;
+  {
+    const int k = kwalk;
+    const int sh = ((p == 0) == (ic < 3)) ? k : -k;
+    const int axis = ic < 3 ? ic : ic - 3;
+    if (axis == 0) {
+      int xd = (int)xa - sh;
+      xd += xd < 0 ? (int)Lh : (xd >= (int)Lh ? -(int)Lh : 0);
+      const int xe = (xd + 1 == (int)Lh) ? 0 : xd + 1;
+      drowA = y * Lh + (uint32_t)xd;
+      drowB = y * Lh + (uint32_t)xe;
+      dpair = !(sh & 1);
+    } else if (axis == 1) {
+      int yd = (int)y - 2 * sh;
+      yd += yd < 0 ? (int)L : (yd >= (int)L ? -(int)L : 0);
+      drowA = (uint32_t)yd * Lh + xa;
+      drowB = drowA + 1;
+    } else {
+      int t = (int)z0 - 2 * sh;
+      t += t < 0 ? (int)L : (t >= (int)L ? -(int)L : 0);
+      zd = (uint32_t)t;
+    }
+  }
+  const size_t dbase = ((size_t)(s * 2 + p) * g.nc + ic) * P * W + grp * VW;
+  uint32_t *q0b = d0 + dbase, *q1b = d1 + dbase;
+
+  auto load_spins = [&](uint32_t t, step_ops<VW> &o) {
+    const uint32_t z = z0 + t, zo = z * plane, rowoff = (y + z + p) & 1;
+    PR::ld(mine + (zo + row) * W, W, o.own, keep);
+    PR::template ld_oth<FLOW>(oth + ((z + 1 == L ? 0 : zo + plane) + row) * W, W, o.up, keep);
+    PR::template ld_oth<FLOW>(oth + (zo + rowN) * W, W, o.vn, keep);
+    PR::template ld_oth<FLOW>(oth + (zo + rowS) * W, W, o.vs, keep);
+    if (FLOW) hint<VW>::ld_co(oth + (zo + (rowoff ? rowXp : rowXm)) * W, o.ext, keep);
+    else hint<VW>::ld_nc(oth + (zo + (rowoff ? rowXp : rowXm)) * W, o.ext, keep);
+  };
+  auto load = [&](uint32_t t, step_ops<VW> &o) {
+    if (ALL) load_spins(t, o);
+    const uint32_t zo = (z0 + t) * plane;
+    uint32_t zt = zd + t;
+    zt -= zt >= L ? L : 0;
+    o.jb2 = ld_u16_keep(jbp + zo + row, keep);
+    const uint32_t sa = (zt * plane + drowA) * W;
+    if (dpair) {
+      PR::ld_na(q0b + sa, W, o.a0, strm);
+      PR::ld_na(q1b + sa, W, o.a1, strm);
+    } else {
+      const uint32_t sb = (zt * plane + drowB) * W;
+      uint32_t x0[VW], x1[VW], y0[VW], y1[VW];
+      hint<VW>::ld_na(q0b + sa, x0, strm);
+      hint<VW>::ld_na(q0b + sb, x1, strm);
+      hint<VW>::ld_na(q1b + sa, y0, strm);
+      hint<VW>::ld_na(q1b + sb, y1, strm);
+#pragma unroll
+      for (int w = 0; w < VW; w++) {
+        o.a0[w] = x0[w]; o.a0[VW + w] = x1[w];
+        o.a1[w] = y0[w]; o.a1[VW + w] = y1[w];
+      }
+    }
+  };
+
+  uint32_t vm[N], v0[N];
+  PR::template ld_oth<FLOW>(oth + ((z0 == 0 ? L - 1 : z0 - 1) * plane + row) * W, W, vm, keep);
+  PR::template ld_oth<FLOW>(oth + (z0 * plane + row) * W, W, v0, keep);
+  step_ops<VW> cur;
+  load(0, cur);
+  uint32_t zdd = zd;
+#pragma unroll(ALL ? 2 : 1)
+  for (uint32_t t = 0; t < (uint32_t)zc; t++) {
+    step_ops<VW> nxt;
+    if (t + 1 < (uint32_t)zc) load(t + 1, nxt);
+    if (pd > 0 && t + (uint32_t)pd < (uint32_t)zc) {
+      uint32_t zf = zdd + (uint32_t)pd;
+      if (zf >= L) zf -= L;
+      prefetch_l2(q0b + (zf * plane + drowA) * W);
+      prefetch_l2(q1b + (zf * plane + drowA) * W);
+    }
+    const uint32_t z = z0 + t, zo = z * plane, rowoff = (y + z + p) & 1;
+    if (!ALL) load_spins(t, cur);
+    const micsa_bonds<2> bonds(cur.jb2, rowoff);
+#pragma unroll
+    for (int site = 0; site < 2; site++) {
+      const uint32_t mC = bonds.column(site), mN = bonds.north(site), mU = bonds.up(site);
+      const uint32_t mB = bonds.beside(site), mS = bonds.south(site), mD = bonds.down(site);
+#pragma unroll
+      for (int w = 0; w < VW; w++) {
+        const int o = site * VW + w;
+        const uint32_t next = site == 0 ? v0[VW + w] : cur.ext[w], prev = site == 0 ? cur.ext[w] : v0[w];
+        const uint32_t sw = cur.own[o], nB = rowoff ? next : prev;
+        const uint32_t f0 = xor3(sw, v0[o], mC), f1 = xor3(sw, cur.vn[o], mN), f2 = xor3(sw, cur.up[o], mU);
+        const uint32_t f3 = xor3(sw, nB, mB), f4 = xor3(sw, cur.vs[o], mS), f5 = xor3(sw, vm[o], mD);
+        const uint32_t j1 = xor3(f0, f1, f2), j2 = maj3(f0, f1, f2);
+        const uint32_t j3 = xor3(f3, f4, f5), j4 = maj3(f3, f4, f5);
+        cur.own[o] = sw ^ isi_update(j1, j2, j3, j4, cur.a0[o], cur.a1[o]);
+      }
+    }
+    PR::st(mine + (zo + row) * W, W, cur.own, keep);
+    const uint32_t sa = (zdd * plane + drowA) * W;
+    if (dpair) {
+      PR::st(q0b + sa, W, cur.a0, strm);
+      PR::st(q1b + sa, W, cur.a1, strm);
+    } else {
+      const uint32_t sb = (zdd * plane + drowB) * W;
+      uint32_t x0[VW], x1[VW], y0[VW], y1[VW];
+#pragma unroll
+      for (int w = 0; w < VW; w++) {
+        x0[w] = cur.a0[w]; x1[w] = cur.a0[VW + w];
+        y0[w] = cur.a1[w]; y1[w] = cur.a1[VW + w];
+      }
+      hint<VW>::st(q0b + sa, x0, strm);
+      hint<VW>::st(q0b + sb, x1, strm);
+      hint<VW>::st(q1b + sa, y0, strm);
+      hint<VW>::st(q1b + sb, y1, strm);
+    }
+#pragma unroll
+    for (int w = 0; w < N; w++) {
+      vm[w] = v0[w];
+      v0[w] = cur.up[w];
+    }
+    zdd = (zdd + 1 == L) ? 0 : zdd + 1;
+    cur = nxt;
+  }
+}
+
 /* ---------------------------------------------------- dataflow sweep */
 /* All 2*nc half-sweeps of one iteration, of every sample, in one launch:
  * the launch boundaries between half-sweeps (each a drain of the whole GPU)
@@ -986,9 +1149,15 @@ k_sweep_dep(const __grid_constant__ micsa_geo g, const __grid_constant__ micsa_f
       y = f.pairs(u);
       x = u - y * f.pairs.d;
     }
-    sweep_block<VW, true, WIDE, false, true, S, LIN, XS, UNR>(
-        g, (int)(job[J_HALF] & 1u), (int)(job[J_HALF] >> 1), job[J_S], job[J_GRP], y, x,
-        job[J_SLAB] * (unsigned)zc, zc, pd, (int)(job[J_WALK] % (unsigned)g.Lh), spin, d0, d1, jb, nullptr, none);
+    if constexpr (LIN && S == 2)
+      sweep_ahead_block<VW, WIDE, true, false>(
+          g, (int)(job[J_HALF] & 1u), (int)(job[J_HALF] >> 1), job[J_S], job[J_GRP], y, x,
+          job[J_SLAB] * (unsigned)zc, zc, pd, (int)(job[J_WALK] % (unsigned)g.Lh), spin, d0, d1, jb);
+    else
+      sweep_block<VW, true, WIDE, false, true, S, LIN, XS, UNR>(
+          g, (int)(job[J_HALF] & 1u), (int)(job[J_HALF] >> 1), job[J_S], job[J_GRP], y, x,
+          job[J_SLAB] * (unsigned)zc, zc, pd, (int)(job[J_WALK] % (unsigned)g.Lh), spin, d0, d1, jb,
+          nullptr, none);
   }
   __syncwarp();
   if ((lin & 31u) == 0) {
@@ -1383,166 +1552,25 @@ k_sweep_async(const micsa_geo g, const int p, const int ic, const int ytiles, co
 
 /* ------------------------------------- sweep with register-pipelined loads */
 /* Operands of one z step of a thread's pair (k_sweep's loads). */
-template <int VW> struct step_ops {
-  uint32_t own[2 * VW], up[2 * VW], vn[2 * VW], vs[2 * VW], a0[2 * VW], a1[2 * VW], ext[VW];
-  uint32_t jb2;
-};
-
 /* The micSA half-sweep of k_sweep with the loads of z step t+1 issued before
  * the arithmetic and stores of step t, so that a thread always has one step
- * of loads in flight while it computes.  Issuing them early is safe: a
- * thread's own spins and demon words are written only by that thread, and
- * the other colour and the couplings are read-only during a half-sweep. */
+ * of loads in flight while it computes (see sweep_ahead_block). */
 template <int VW, bool WIDE, int MINB>
 __global__ void __launch_bounds__(TPB, MINB)
 k_sweep_pipe(const micsa_geo g, const int p, const int ic, const int ytiles, const int G,
              const int zc, const int pd, uint32_t *__restrict__ spin, uint32_t *__restrict__ d0,
              uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb,
              const int *__restrict__ walk) {
-  constexpr int N = 2 * VW;
-  using PR = pairs<VW, WIDE>;
   grid_dependency_sync();
-  const uint32_t L = g.L, Lh = g.Lh, W = g.W;
   const uint32_t by = blockIdx.y;
   const uint32_t tile = by % ytiles, sg = by / ytiles;
   const uint32_t s = sg / G, grp = sg % G;
   /* the walk and the run flag are loaded together: one round trip */
   const int kwalk = __ldg(walk + s);
-  if (micsa_frozen(g, (int)s)) return;
-  const uint32_t y = tile * blockDim.y + threadIdx.y;
-  if (y >= L) return;
-  const uint32_t xa = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
-  const uint32_t plane = L * Lh;
-  const uint32_t z0 = blockIdx.z * zc;
-  const uint32_t row = y * Lh + xa;
-  const uint32_t rowN = (y + 1 == L) ? xa : row + Lh;
-  const uint32_t rowS = (y == 0) ? row + (L - 1) * Lh : row - Lh;
-  const uint32_t rowXp = (xa + 2 == Lh) ? row + 2 - Lh : row + 2;
-  const uint32_t rowXm = (xa == 0) ? row + Lh - 1 : row - 1;
-  const size_t P = (size_t)g.P;
-  uint32_t *mine = spin + (size_t)(s * 2 + p) * P * W + grp * VW;
-  const uint32_t *oth = spin + (size_t)(s * 2 + (p ^ 1)) * P * W + grp * VW;
-  const uint8_t *jbp = jb + (size_t)(s * 2 + p) * P;
-  const uint64_t keep = l2_keep(), strm = l2_stream();
-
-  uint32_t drowA = row, drowB = row + 1, zd = z0;
-  bool dpair = true;
-  {
-    const int k = kwalk;
-    const int sh = ((p == 0) == (ic < 3)) ? k : -k;
-    const int axis = ic < 3 ? ic : ic - 3;
-    if (axis == 0) {
-      int xd = (int)xa - sh;
-      xd += xd < 0 ? (int)Lh : (xd >= (int)Lh ? -(int)Lh : 0);
-      const int xe = (xd + 1 == (int)Lh) ? 0 : xd + 1;
-      drowA = y * Lh + (uint32_t)xd;
-      drowB = y * Lh + (uint32_t)xe;
-      dpair = !(sh & 1);
-    } else if (axis == 1) {
-      int yd = (int)y - 2 * sh;
-      yd += yd < 0 ? (int)L : (yd >= (int)L ? -(int)L : 0);
-      drowA = (uint32_t)yd * Lh + xa;
-      drowB = drowA + 1;
-    } else {
-      int t = (int)z0 - 2 * sh;
-      t += t < 0 ? (int)L : (t >= (int)L ? -(int)L : 0);
-      zd = (uint32_t)t;
-    }
-  }
-  const size_t dbase = ((size_t)(s * 2 + p) * g.nc + ic) * P * W + grp * VW;
-  uint32_t *q0b = d0 + dbase, *q1b = d1 + dbase;
-
-  auto load = [&](uint32_t t, step_ops<VW> &o) {
-    const uint32_t z = z0 + t, zo = z * plane, rowoff = (y + z + p) & 1;
-    uint32_t zt = zd + t;
-    zt -= zt >= L ? L : 0;
-    PR::ld(mine + (zo + row) * W, W, o.own, keep);
-    PR::ld_nc(oth + ((z + 1 == L ? 0 : zo + plane) + row) * W, W, o.up, keep);
-    PR::ld_nc(oth + (zo + rowN) * W, W, o.vn, keep);
-    PR::ld_nc(oth + (zo + rowS) * W, W, o.vs, keep);
-    hint<VW>::ld_nc(oth + (zo + (rowoff ? rowXp : rowXm)) * W, o.ext, keep);
-    o.jb2 = ld_u16_keep(jbp + zo + row, keep);
-    const uint32_t sa = (zt * plane + drowA) * W;
-    if (dpair) {
-      PR::ld_na(q0b + sa, W, o.a0, strm);
-      PR::ld_na(q1b + sa, W, o.a1, strm);
-    } else {
-      const uint32_t sb = (zt * plane + drowB) * W;
-      uint32_t x0[VW], x1[VW], y0[VW], y1[VW];
-      hint<VW>::ld_na(q0b + sa, x0, strm);
-      hint<VW>::ld_na(q0b + sb, x1, strm);
-      hint<VW>::ld_na(q1b + sa, y0, strm);
-      hint<VW>::ld_na(q1b + sb, y1, strm);
-#pragma unroll
-      for (int w = 0; w < VW; w++) {
-        o.a0[w] = x0[w]; o.a0[VW + w] = x1[w];
-        o.a1[w] = y0[w]; o.a1[VW + w] = y1[w];
-      }
-    }
-  };
-
-  uint32_t vm[N], v0[N];
-  PR::ld_nc(oth + ((z0 == 0 ? L - 1 : z0 - 1) * plane + row) * W, W, vm, keep);
-  PR::ld_nc(oth + (z0 * plane + row) * W, W, v0, keep);
-  step_ops<VW> cur;
-  load(0, cur);
-  uint32_t zdd = zd;
-#pragma unroll 2
-  for (uint32_t t = 0; t < (uint32_t)zc; t++) {
-    step_ops<VW> nxt;
-    if (t + 1 < (uint32_t)zc) load(t + 1, nxt);
-    if (pd > 0 && t + (uint32_t)pd < (uint32_t)zc) {
-      uint32_t zf = zdd + (uint32_t)pd;
-      if (zf >= L) zf -= L;
-      prefetch_l2(q0b + (zf * plane + drowA) * W);
-      prefetch_l2(q1b + (zf * plane + drowA) * W);
-    }
-    const uint32_t z = z0 + t, zo = z * plane, rowoff = (y + z + p) & 1;
-#pragma unroll
-    for (int site = 0; site < 2; site++) {
-      const uint32_t jb6 = (cur.jb2 >> (8 * site)) & 0xffu;
-      const uint32_t mE = jmask(jb6, 0), mN = jmask(jb6, 1), mU = jmask(jb6, 2);
-      const uint32_t mO = jmask(jb6, 3), mS = jmask(jb6, 4), mD = jmask(jb6, 5);
-#pragma unroll
-      for (int w = 0; w < VW; w++) {
-        const int o = site * VW + w;
-        const uint32_t cA = v0[w], cB = v0[VW + w], ex = cur.ext[w];
-        const uint32_t nE = site == 0 ? (rowoff ? cB : cA) : (rowoff ? ex : cB);
-        const uint32_t nO = site == 0 ? (rowoff ? cA : ex) : (rowoff ? cB : cA);
-        const uint32_t sw = cur.own[o];
-        const uint32_t f0 = xor3(sw, nE, mE), f1 = xor3(sw, cur.vn[o], mN), f2 = xor3(sw, cur.up[o], mU);
-        const uint32_t f3 = xor3(sw, nO, mO), f4 = xor3(sw, cur.vs[o], mS), f5 = xor3(sw, vm[o], mD);
-        const uint32_t j1 = xor3(f0, f1, f2), j2 = maj3(f0, f1, f2);
-        const uint32_t j3 = xor3(f3, f4, f5), j4 = maj3(f3, f4, f5);
-        cur.own[o] = sw ^ isi_update(j1, j2, j3, j4, cur.a0[o], cur.a1[o]);
-      }
-    }
-    PR::st(mine + (zo + row) * W, W, cur.own, keep);
-    const uint32_t sa = (zdd * plane + drowA) * W;
-    if (dpair) {
-      PR::st(q0b + sa, W, cur.a0, strm);
-      PR::st(q1b + sa, W, cur.a1, strm);
-    } else {
-      const uint32_t sb = (zdd * plane + drowB) * W;
-      uint32_t x0[VW], x1[VW], y0[VW], y1[VW];
-#pragma unroll
-      for (int w = 0; w < VW; w++) {
-        x0[w] = cur.a0[w]; x1[w] = cur.a0[VW + w];
-        y0[w] = cur.a1[w]; y1[w] = cur.a1[VW + w];
-      }
-      hint<VW>::st(q0b + sa, x0, strm);
-      hint<VW>::st(q0b + sb, x1, strm);
-      hint<VW>::st(q1b + sa, y0, strm);
-      hint<VW>::st(q1b + sb, y1, strm);
-    }
-#pragma unroll
-    for (int w = 0; w < N; w++) {
-      vm[w] = v0[w];
-      v0[w] = cur.up[w];
-    }
-    zdd = (zdd + 1 == L) ? 0 : zdd + 1;
-    cur = nxt;
-  }
+  if (micsa_frozen(g, s)) return;
+  sweep_ahead_block<VW, WIDE, false, true>(g, p, ic, s, grp, tile * blockDim.y + threadIdx.y,
+                                           blockIdx.x * blockDim.x + threadIdx.x, blockIdx.z * zc, zc,
+                                           pd, kwalk, spin, d0, d1, jb);
 }
 
 /* ------------------------------------------------------ Philox + LUT bits */
