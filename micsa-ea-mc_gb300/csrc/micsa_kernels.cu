@@ -683,13 +683,13 @@ k_sweep(const micsa_geo g, const int p, const int ic, const int ytiles, const in
                                               zc, pd, kwalk, spin, d0, d1, jb, rnd, tm);
 }
 
-template <int VW> struct step_ops {
-  uint32_t own[2 * VW], up[2 * VW], vn[2 * VW], vs[2 * VW], a0[2 * VW], a1[2 * VW], ext[VW];
-  uint32_t jb2;
+template <int VW, int S> struct step_ops {
+  uint32_t own[S * VW], up[S * VW], vn[S * VW], vs[S * VW], a0[S * VW], a1[S * VW], ext[VW];
+  uint32_t jbs;
 };
 
-/* One thread's columns of a half-sweep, as in sweep_block (pairs, direct
- * loads), with loads of z step t+1 issued before the arithmetic and stores of
+/* One thread's columns of a half-sweep, as in sweep_block (direct loads, S
+ * sites), with loads of z step t+1 issued before the arithmetic and stores of
  * step t: all of them (ALL), or its demon words and couplings only, which
  * takes 9 instead of 27 registers: pairs of two-word sites fit 64 registers
  * without spills.  The dataflow sweep's tiles use the latter (us per
@@ -699,22 +699,22 @@ template <int VW> struct step_ops {
  * is safe: a thread's own spins and demon words are written only by that
  * thread, the couplings are constant, and in a launch of one half-sweep (not
  * FLOW) the other colour is read-only. */
-template <int VW, bool WIDE, bool FLOW, bool ALL>
+template <int VW, bool WIDE, bool FLOW, bool ALL, int S = 2>
 __device__ __forceinline__ void sweep_ahead_block(
     const micsa_geo &g, const int p, const int ic, const uint32_t s, const uint32_t grp,
-    const uint32_t y, const uint32_t pair, const uint32_t z0, const int zc, const int pd,
+    const uint32_t y, const uint32_t unit, const uint32_t z0, const int zc, const int pd,
     const int kwalk, uint32_t *__restrict__ spin, uint32_t *__restrict__ d0,
     uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb) {
-  constexpr int N = 2 * VW;
-  using PR = pairs<VW, WIDE>;
+  constexpr int N = S * VW;
+  using PR = typename sites_io<VW, WIDE, S>::type;
   const uint32_t L = g.L, Lh = g.Lh, W = WIDE ? (uint32_t)VW : (uint32_t)g.W;
   if (y >= L) return;
-  const uint32_t xa = 2 * pair;
+  const uint32_t xa = S * unit;
   const uint32_t plane = L * Lh;
   const uint32_t row = y * Lh + xa;
   const uint32_t rowN = (y + 1 == L) ? xa : row + Lh;
   const uint32_t rowS = (y == 0) ? row + (L - 1) * Lh : row - Lh;
-  const uint32_t rowXp = (xa + 2 == Lh) ? row + 2 - Lh : row + 2;
+  const uint32_t rowXp = (xa + S == Lh) ? row + S - Lh : row + S;
   const uint32_t rowXm = (xa == 0) ? row + Lh - 1 : row - 1;
   const size_t P = (size_t)g.P;
   uint32_t *mine = spin + (size_t)(s * 2 + p) * P * W + grp * VW;
@@ -734,7 +734,7 @@ __device__ __forceinline__ void sweep_ahead_block(
       const int xe = (xd + 1 == (int)Lh) ? 0 : xd + 1;
       drowA = y * Lh + (uint32_t)xd;
       drowB = y * Lh + (uint32_t)xe;
-      dpair = !(sh & 1);
+      dpair = !(sh & (S - 1));
     } else if (axis == 1) {
       int yd = (int)y - 2 * sh;
       yd += yd < 0 ? (int)L : (yd >= (int)L ? -(int)L : 0);
@@ -749,7 +749,7 @@ __device__ __forceinline__ void sweep_ahead_block(
   const size_t dbase = ((size_t)(s * 2 + p) * g.nc + ic) * P * W + grp * VW;
   uint32_t *q0b = d0 + dbase, *q1b = d1 + dbase;
 
-  auto load_spins = [&](uint32_t t, step_ops<VW> &o) {
+  auto load_spins = [&](uint32_t t, step_ops<VW, S> &o) {
     const uint32_t z = z0 + t, zo = z * plane, rowoff = (y + z + p) & 1;
     PR::ld(mine + (zo + row) * W, W, o.own, keep);
     PR::template ld_oth<FLOW>(oth + ((z + 1 == L ? 0 : zo + plane) + row) * W, W, o.up, keep);
@@ -758,16 +758,25 @@ __device__ __forceinline__ void sweep_ahead_block(
     if (FLOW) hint<VW>::ld_co(oth + (zo + (rowoff ? rowXp : rowXm)) * W, o.ext, keep);
     else hint<VW>::ld_nc(oth + (zo + (rowoff ? rowXp : rowXm)) * W, o.ext, keep);
   };
-  auto load = [&](uint32_t t, step_ops<VW> &o) {
+  auto load = [&](uint32_t t, step_ops<VW, S> &o) {
     if (ALL) load_spins(t, o);
     const uint32_t zo = (z0 + t) * plane;
     uint32_t zt = zd + t;
     zt -= zt >= L ? L : 0;
-    o.jb2 = ld_u16_keep(jbp + zo + row, keep);
+    o.jbs = S == 4 ? ld_u32_keep(jbp + zo + row, keep) : ld_u16_keep(jbp + zo + row, keep);
     const uint32_t sa = (zt * plane + drowA) * W;
     if (dpair) {
       PR::ld_na(q0b + sa, W, o.a0, strm);
       PR::ld_na(q1b + sa, W, o.a1, strm);
+    } else if constexpr (S == 4) { /* four single words, each wrapped along the row */
+      const uint32_t xd = drowA % Lh, rbase = zt * plane + (drowA - xd);
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        uint32_t xk = xd + k;
+        xk -= xk >= Lh ? Lh : 0;
+        o.a0[k] = ld_na_u32(q0b + rbase + xk, strm);
+        o.a1[k] = ld_na_u32(q1b + rbase + xk, strm);
+      }
     } else {
       const uint32_t sb = (zt * plane + drowB) * W;
       uint32_t x0[VW], x1[VW], y0[VW], y1[VW];
@@ -786,12 +795,12 @@ __device__ __forceinline__ void sweep_ahead_block(
   uint32_t vm[N], v0[N];
   PR::template ld_oth<FLOW>(oth + ((z0 == 0 ? L - 1 : z0 - 1) * plane + row) * W, W, vm, keep);
   PR::template ld_oth<FLOW>(oth + (z0 * plane + row) * W, W, v0, keep);
-  step_ops<VW> cur;
+  step_ops<VW, S> cur;
   load(0, cur);
   uint32_t zdd = zd;
 #pragma unroll(ALL ? 2 : 1)
   for (uint32_t t = 0; t < (uint32_t)zc; t++) {
-    step_ops<VW> nxt;
+    step_ops<VW, S> nxt;
     if (t + 1 < (uint32_t)zc) load(t + 1, nxt);
     if (pd > 0 && t + (uint32_t)pd < (uint32_t)zc) {
       uint32_t zf = zdd + (uint32_t)pd;
@@ -801,15 +810,16 @@ __device__ __forceinline__ void sweep_ahead_block(
     }
     const uint32_t z = z0 + t, zo = z * plane, rowoff = (y + z + p) & 1;
     if (!ALL) load_spins(t, cur);
-    const micsa_bonds<2> bonds(cur.jb2, rowoff);
+    const micsa_bonds<S> bonds(cur.jbs, rowoff);
 #pragma unroll
-    for (int site = 0; site < 2; site++) {
+    for (int site = 0; site < S; site++) {
       const uint32_t mC = bonds.column(site), mN = bonds.north(site), mU = bonds.up(site);
       const uint32_t mB = bonds.beside(site), mS = bonds.south(site), mD = bonds.down(site);
 #pragma unroll
       for (int w = 0; w < VW; w++) {
         const int o = site * VW + w;
-        const uint32_t next = site == 0 ? v0[VW + w] : cur.ext[w], prev = site == 0 ? cur.ext[w] : v0[w];
+        const uint32_t next = site + 1 < S ? v0[(site + 1 < S ? site + 1 : 0) * VW + w] : cur.ext[w];
+        const uint32_t prev = site > 0 ? v0[(site > 0 ? site - 1 : 0) * VW + w] : cur.ext[w];
         const uint32_t sw = cur.own[o], nB = rowoff ? next : prev;
         const uint32_t f0 = xor3(sw, v0[o], mC), f1 = xor3(sw, cur.vn[o], mN), f2 = xor3(sw, cur.up[o], mU);
         const uint32_t f3 = xor3(sw, nB, mB), f4 = xor3(sw, cur.vs[o], mS), f5 = xor3(sw, vm[o], mD);
@@ -823,6 +833,15 @@ __device__ __forceinline__ void sweep_ahead_block(
     if (dpair) {
       PR::st(q0b + sa, W, cur.a0, strm);
       PR::st(q1b + sa, W, cur.a1, strm);
+    } else if constexpr (S == 4) {
+      const uint32_t xd = drowA % Lh, rbase = zdd * plane + (drowA - xd);
+#pragma unroll
+      for (int k = 0; k < N; k++) {
+        uint32_t xk = xd + k;
+        xk -= xk >= Lh ? Lh : 0;
+        st_u32(q0b + rbase + xk, cur.a0[k], strm);
+        st_u32(q1b + rbase + xk, cur.a1[k], strm);
+      }
     } else {
       const uint32_t sb = (zdd * plane + drowB) * W;
       uint32_t x0[VW], x1[VW], y0[VW], y1[VW];
@@ -1070,8 +1089,8 @@ struct micsa_flow_plan {
  * and no idle lanes where a row's units do not divide the block (L=160: 25
  * tiles a slab of 8 full warps instead of 27 of 7.5; 386 -> 371 us at 8
  * planes).  Four one-word sites a thread (S = 4) halve the tiles of
- * 32-replica lattices (L=104, 3 samples: 106 us, 110 by pairs; L=128, 1
- * sample: 73, 78 by pairs).
+ * 32-replica lattices, which pays with few samples (L=128, 1 sample: 66 us,
+ * 67.5 by pairs; L=104, 3 samples: 99, 96.5 by pairs).
  *
  * The tile's values go through shared memory and are read where they are
  * used, so that none of them stays in a register across the sweep body
@@ -1149,8 +1168,8 @@ k_sweep_dep(const __grid_constant__ micsa_geo g, const __grid_constant__ micsa_f
       y = f.pairs(u);
       x = u - y * f.pairs.d;
     }
-    if constexpr (LIN && S == 2)
-      sweep_ahead_block<VW, WIDE, true, false>(
+    if constexpr (LIN)
+      sweep_ahead_block<VW, WIDE, true, false, S>(
           g, (int)(job[J_HALF] & 1u), (int)(job[J_HALF] >> 1), job[J_S], job[J_GRP], y, x,
           job[J_SLAB] * (unsigned)zc, zc, pd, (int)(job[J_WALK] % (unsigned)g.Lh), spin, d0, d1, jb);
     else
