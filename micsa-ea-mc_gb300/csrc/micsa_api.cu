@@ -1155,15 +1155,18 @@ int micsa_refresh_wait(micsa_ctx *ctx) {
 namespace {
 
 /* Whether a refresh asked for ahead is drawn at once on the side stream or
- * recorded and drawn in place on the context's stream at the commit.  A
- * context whose sweep is the dataflow kernel fills the GPU, and a draw
- * beside it slows both: L=160 x 2 samples, a 20-iteration job with 6
- * refreshes took 59.4 ms drawn ahead (whose commit also copies the demon
- * planes) against 56.6 ms drawn in place.  MICSA_REFRESH_AHEAD=1 keeps the
+ * recorded and drawn in place on the context's stream at the commit.  The
+ * dataflow kernel of a large lattice fills the GPU, and a draw beside it
+ * slows both: L=160 x 2 samples, a 20-iteration job with 6 refreshes took
+ * 59.4 ms drawn ahead (whose commit also copies the demon planes) against
+ * 56.6 ms drawn in place.  Below L=128 drawing ahead stays 1 to 2% faster
+ * (64-iteration jobs: L=64 x 4 11.15 against 11.40 ms, L=48 x 12 14.55
+ * against 14.89, L=96 x 4 of 32 replicas 17.56 against 17.67).
+ * MICSA_REFRESH_AHEAD=1 keeps the
  * side stream for every context, =0 defers for every context. */
 bool refresh_deferred(const micsa_ctx *ctx) {
   if (const char *e = getenv("MICSA_REFRESH_AHEAD")) return atoi(e) == 0;
-  return ctx->g.flow != 0;
+  return ctx->g.flow && ctx->g.L >= 128;
 }
 
 int refresh_occ() {
