@@ -32,13 +32,15 @@
  *                        choice for its shape
  *   MICSA_RESIDENT=0     keep L <= 32 on the per-half-sweep kernels
  *   MICSA_RESIDENT_CTAS=c  blocks per cluster of the resident kernel (1, 2, 4 or 8
- *                        where the shape has that size), for calls of any length
+ *                        where the shape has that size), for calls of any length,
+ *                        each in one launch
  *   MICSA_PDL=0          plain launches instead of programmatic dependent launch
  *   MICSA_REFRESH_WPS=n  segment length of the GPU demon refresh, in words
  *   MICSA_REFRESH_OCC=1  the refresh kernel without its register budget
  *   MICSA_REFRESH_AHEAD=0|1  refreshes asked for ahead: drawn in place at the
  *                        commit (0) or at once on the side stream (1); default:
- *                        in place for contexts on the dataflow sweep
+ *                        in place for contexts on the dataflow sweep from
+ *                        L = 128
  *   MICSA_FLOW_ITERS=k   iterations per dataflow launch, with a pinned shape
  *   MICSA_SWEEP_PERS=1   the dataflow sweep's persistent form, with a pinned shape
  *   MICSA_FLOW_HALF=1    half-height dataflow tiles, with a pinned shape
