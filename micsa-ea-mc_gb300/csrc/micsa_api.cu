@@ -446,14 +446,22 @@ int autotune(micsa_ctx *ctx) {
    * kernels need: with the dataflow sweep at every size the served stream
    * fell from 5.41 to 4.66 anneals/s and the batched one from 92.6 to 87.7.
    * Theirs try it only for L >= 128 (where they would run few samples); a
-   * context of its own tries it at every L (us per iteration, against the
-   * best of the other forms: L=64, 8 samples x 64 replicas 87 against 102;
-   * L=96, 2 x 64: 84 against 99; L=104, 3 x 32: 103 against 123; L=48,
-   * 32 x 64: 143 against 151).  MICSA_SWEEP_FLOW=0 leaves it out everywhere. */
-  const char *ef0 = getenv("MICSA_SWEEP_FLOW");
-  const bool try_flow = !(ef0 && !strcmp(ef0, "0")) && (g.L >= 128 || !ctx->shared);
+   * context of its own tries it below that too if it fills the GPU by itself:
+   * 2.25 z planes or more for each thread that the GPU holds (us per
+   * iteration, against the best of the other forms: L=64, 8 samples x 64
+   * replicas 85 against 102; L=96, 2 x 64: 80 against 99; L=104, 3 x 32: 97
+   * against 116; L=48, 32 x 64: 138 against 151).  Three such contexts at
+   * work together lose nothing by it (L=64, 8 x 64 84 against 84 per
+   * context; L=96, 2 x 64 80 against 84; L=48, 16 x 64 83 against 78), three
+   * smaller ones would (L=64, 4 x 64: 57 against 43).  MICSA_SWEEP_FLOW=0
+   * leaves it out everywhere. */
   int nsm = 0;
   MICSA_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->cfg.device));
+  const int groups = g.W % 4 == 0 ? g.W / 4 : (g.W % 2 == 0 ? g.W / 2 : g.W);
+  const double planes = (double)g.L * g.L * g.Lh / 2 * groups * g.ns; /* of all threads' columns */
+  const char *ef0 = getenv("MICSA_SWEEP_FLOW");
+  const bool try_flow = !(ef0 && !strcmp(ef0, "0")) &&
+                        (g.L >= 128 || (!ctx->shared && planes >= 2.25 * nsm * 1024));
   const int reps = 3;
   /* sample orders: all samples per launch, or sample-major.  Launches per
    * group of 2 to 8 samples (MICSA_SWEEP_SPLIT=k) are not timed: alone they
@@ -520,7 +528,7 @@ int autotune(micsa_ctx *ctx) {
          * fastest depth had 0.84 (L=64, 8 samples) to 1.3 (L=160) of the
          * blocks at all sizes tried, so the others are not timed */
         const double tiles = (double)((g.L * g.Lh / (tm == 7 ? 4 : 2) + 255) / 256) *
-                             (g.W % 4 == 0 ? g.W / 4 : (g.W % 2 == 0 ? g.W / 2 : g.W)) * (g.L / zc) * (sp ? 1 : g.ns);
+                             groups * (g.L / zc) * (sp ? 1 : g.ns);
         const double held = (double)nsm * (g.W % 4 ? (oc ? 4 : 3) : 2);
         const bool last = c + 1 == nfz;
         if (tiles < 0.7 * held || (tiles > 2.2 * held && !last)) continue;
