@@ -474,7 +474,8 @@ int autotune(micsa_ctx *ctx) {
    * 3 loads pipelined one step ahead in registers (register budget for 3 or 2
    * blocks per SM instead of 3 or 4), 4 direct loads in one dataflow launch
    * per iteration (split: its tiles sample-major or half-sweep-major), 5
-   * direct loads with four one-word sites per thread (W = 1) */
+   * direct loads with four one-word sites per thread (W = 1), 7 the dataflow
+   * launch with those (both in tiles of consecutive units, tw = 2) */
   /* mean ms per half-sweep of the shape in g (sample order sp): reps replays
    * of a graph of one iteration (16 for the dataflow sweep) in their launch
    * order, as micsa_iterate runs them -- timed launch by launch, small
