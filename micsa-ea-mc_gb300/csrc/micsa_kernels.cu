@@ -228,9 +228,9 @@ __device__ __forceinline__ uint32_t ld_u16_keep(const uint8_t *a, uint64_t pol) 
   return v;
 }
 
-/* The two sites of a pair: with one word group per site (WIDE, G = 1) their
- * words are adjacent and move as one vector; otherwise they are W words
- * apart and move as two vectors. */
+/* The two sites of a pair: with one word group per site (WIDE, only where
+ * W = VW) their words are adjacent and move as one vector; otherwise they are
+ * W words apart and move as two vectors. */
 template <int VW, bool WIDE> struct pairs {
   static constexpr int N = 2 * VW;
   static __device__ __forceinline__ void cat(uint32_t (&o)[N], const uint32_t (&a)[VW],
@@ -2879,8 +2879,9 @@ cudaError_t micsa_launch_sweep_multi(const micsa_multi_args &a, int occ, unsigne
   for (int i = 1; i < a.n; i++)
     if (a.gr[i].g.W != W) return cudaErrorInvalidValue;
   const dim3 grid(a.total), block(MTPB);
-  /* the word vector of one site: 4, 2 or 1 words; one group of them (WIDE)
-   * when it is all of a site's words */
+  /* the word vector of one site: 4, 2 or 1 words; WIDE only where that vector
+   * is all of a site's words (W = VW): the body then takes VW for the words
+   * per site and loads two sites as one run */
   if (W % 4 == 0) {
     if (W == 4) k_sweep_multi<4, true, 4><<<grid, block, 0, st>>>(a, ctl);
     else k_sweep_multi<4, false, 4><<<grid, block, 0, st>>>(a, ctl);
@@ -2892,9 +2893,11 @@ cudaError_t micsa_launch_sweep_multi(const micsa_multi_args &a, int occ, unsigne
     } else {
       k_sweep_multi<2, false, 6><<<grid, block, 0, st>>>(a, ctl);
     }
-  } else {
+  } else if (W == 1) {
     if (occ == 8) k_sweep_multi<1, true, 8><<<grid, block, 0, st>>>(a, ctl);
     else k_sweep_multi<1, true, 6><<<grid, block, 0, st>>>(a, ctl);
+  } else { /* 3, 5, ... groups of one word (at 64 registers, occ = 8, it would spill) */
+    k_sweep_multi<1, false, 6><<<grid, block, 0, st>>>(a, ctl);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
