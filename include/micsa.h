@@ -104,8 +104,9 @@ int micsa_set_lut(micsa_ctx *ctx, const void *lut, size_t bytes);
 int micsa_upload_couplings(micsa_ctx *ctx, int sample, const uint64_t *J);
 /* Spins of one sample, reference layout (CopyDataOnDevice, main.cu:429-434).
  * Here and for the demons: when both host buffers are page-locked and mapped
- * the conversion kernel reads them directly across the host link; other
- * buffers go through a device staging buffer.  The results are the same. */
+ * (from the first word to the last) and 8-byte aligned, the conversion kernel
+ * reads them directly across the host link; other buffers go through a device
+ * staging buffer.  The results are the same. */
 int micsa_upload_spins(micsa_ctx *ctx, int sample, const uint64_t *even,
                        const uint64_t *odd);
 /* Demons of one sample, CPUwalker layout; resets that sample's demon walk

@@ -105,12 +105,15 @@ int fail(micsa_ctx *c, int code, const char *fmt, ...) {
   return code;
 }
 
+/* a refused call's error is reported here and not left for the next call's check */
 #define MICSA_CK(call)                                                              \
   do {                                                                              \
     cudaError_t e_ = (call);                                                        \
-    if (e_ != cudaSuccess)                                                          \
+    if (e_ != cudaSuccess) {                                                        \
+      (void)cudaGetLastError();                                                     \
       return fail(ctx, MICSA_ERR_CUDA, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), \
                   __FILE__, __LINE__);                                              \
+    }                                                                               \
   } while (0)
 
 struct sizes {
@@ -172,18 +175,27 @@ int ensure_stage(micsa_ctx *ctx) {
   return MICSA_OK;
 }
 
-/* The device address of a caller's host buffer that kernels may read and write
- * directly (page-locked and mapped, as cudaHostAlloc and mapped registered
- * memory are), else nullptr.  Transfers from and to such a buffer convert
- * straight across the host link: one pass at link speed instead of a copy
- * and a conversion one after the other through the staging buffer. */
-uint64_t *device_view(const uint64_t *p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    (void)cudaGetLastError(); /* not a pointer the runtime knows: the staged path */
-    return nullptr;
+/* The device address of a caller's host buffer of n words that kernels may
+ * read and write directly (page-locked and mapped, as cudaHostAlloc and mapped
+ * registered memory are), else nullptr.  Transfers from and to such a buffer
+ * convert straight across the host link: one pass at link speed instead of a
+ * copy and a conversion one after the other through the staging buffer, which
+ * also takes what a kernel could not address: a buffer off its 8-byte
+ * alignment, or one of which only the beginning is page-locked. */
+uint64_t *device_view(const uint64_t *p, int64_t n) {
+  if ((uintptr_t)p % sizeof(uint64_t)) return nullptr;
+  const uint64_t *ends[2] = {p, p + (n - 1)};
+  char *at[2];
+  for (int k = 0; k < 2; k++) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, ends[k]) != cudaSuccess) {
+      (void)cudaGetLastError(); /* not a pointer the runtime knows */
+      return nullptr;
+    }
+    if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+    at[k] = (char *)a.devicePointer;
   }
-  return a.type == cudaMemoryTypeHost ? (uint64_t *)a.devicePointer : nullptr;
+  return at[1] - at[0] == (const char *)ends[1] - (const char *)ends[0] ? (uint64_t *)at[0] : nullptr;
 }
 
 int ready_for_sweeps(micsa_ctx *ctx, int need_demons) {
@@ -1084,7 +1096,7 @@ int micsa_upload_spins(micsa_ctx *ctx, int sample, const uint64_t *even, const u
   if (rc || (rc = set_device(ctx))) return rc;
   const micsa_geo &g = ctx->g;
   const int64_t n = g.H * g.nr;
-  const uint64_t *src[2] = {device_view(even), device_view(odd)};
+  const uint64_t *src[2] = {device_view(even, n), device_view(odd, n)};
   if (!src[0] || !src[1]) {
     if ((rc = ensure_stage(ctx))) return rc;
     MICSA_CK(cudaMemcpyAsync(ctx->stage, even, 8 * n, cudaMemcpyHostToDevice, ctx->stream));
@@ -1107,7 +1119,7 @@ int micsa_upload_demons(micsa_ctx *ctx, int sample, const uint64_t *w0, const ui
   const micsa_geo &g = ctx->g;
   const int planes = 2 * g.nc;
   const int64_t n = planes * g.H * g.nr, o = (int64_t)sample * planes * g.P * g.W;
-  const uint64_t *src[2] = {device_view(w0), device_view(w1)};
+  const uint64_t *src[2] = {device_view(w0, n), device_view(w1, n)};
   if (src[0] && src[1]) {
     MICSA_CK(micsa_launch_from_ref(g, planes, 2 * planes, src[0], src[1], ctx->dem0 + o, ctx->dem1 + o,
                                    ctx->stream));
@@ -1511,7 +1523,7 @@ int micsa_download_spins(micsa_ctx *ctx, int sample, uint64_t *even, uint64_t *o
   if (rc || (rc = set_device(ctx))) return rc;
   const micsa_geo &g = ctx->g;
   const int64_t n = g.H * g.nr;
-  uint64_t *dv[2] = {device_view(even), device_view(odd)};
+  uint64_t *dv[2] = {device_view(even, n), device_view(odd, n)};
   const bool direct = dv[0] && dv[1];
   if (!direct && (rc = ensure_stage(ctx))) return rc;
   const uint32_t *src = ctx->spin + (int64_t)sample * 2 * g.P * g.W;
@@ -1536,7 +1548,7 @@ int micsa_download_demons(micsa_ctx *ctx, int sample, uint64_t *w0, uint64_t *w1
   const int64_t n = planes * g.H * g.nr, o = (int64_t)sample * planes * g.P * g.W;
   const uint32_t *src[2] = {ctx->dem0 + o, ctx->dem1 + o};
   uint64_t *dst[2] = {w0, w1};
-  uint64_t *dv[2] = {device_view(w0), device_view(w1)};
+  uint64_t *dv[2] = {device_view(w0, n), device_view(w1, n)};
   if (dv[0] && dv[1]) {
     MICSA_CK(micsa_launch_to_ref(g, planes, 2 * planes, ctx->walk, sample, src[0], src[1], dv[0], dv[1],
                                  ctx->stream));
