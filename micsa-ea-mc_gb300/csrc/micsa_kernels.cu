@@ -2242,6 +2242,8 @@ static cudaError_t sweep_vw(const micsa_geo &g, int p, int ic, bool micsa, uint3
   const bool tma = micsa && tm && tm->ok && g.tma && G == 1 && g.L % ty == 0 && zc <= 4 &&
                    tm->ty == ty && tm->box_w >= 2 * tx * VW;
   const size_t smem = tma ? (size_t)2 * zc * ty * tm->box_w * 4 + (size_t)zc * 8 : 0;
+  /* ... of any lattice: ty * box_w <= (TPB / tx) * (2 * tx * VW + 4) words, tx >= 1, zc <= 4 */
+  constexpr size_t most = 2 * 4 * TPB * (2 * VW + 4) * 4 + 4 * 8;
   if (VW == 2 && micsa && g.async && G == 1 && !tma) {
     const size_t sb = (size_t)2 * ASYNC_ITEMS * TPB * 16;
     cudaError_t e;
@@ -2291,9 +2293,10 @@ static cudaError_t sweep_vw(const micsa_geo &g, int p, int ic, bool micsa, uint3
 #define MICSA_SWEEP(M, WD, B, T)                                                                  \
   do {                                                                                            \
     if (T && smem > 48 * 1024) {                                                                  \
+      /* the limit is the function's: the same value for every context */                         \
       const cudaError_t e_ = cudaFuncSetAttribute(k_sweep<VW, M, WD, B, T>,                       \
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                                  (int)smem);                                     \
+                                                  (int)most);                                     \
       if (e_ != cudaSuccess) return e_;                                                           \
     }                                                                                             \
     const cudaError_t l_ = launch_sweep(g, k_sweep<VW, M, WD, B, T>, grid, block, smem, st, g, p, \
@@ -2607,8 +2610,10 @@ cudaError_t micsa_launch_overlap(const micsa_geo &g, const uint32_t *spin, unsig
   if (tiles < 1) tiles = 1;
   const size_t smem = sizeof(uint32_t) * OV_PITCH * (size_t)(g.L + g.Lh);
   if (smem > 48 * 1024) {
+    /* the limit is the function's, not the launch's: always that of the largest
+     * lattice (L = 888, 176 KB), so that threads with other L cannot lower it */
     const cudaError_t e = cudaFuncSetAttribute(k_overlap, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
+                                               (int)(sizeof(uint32_t) * OV_PITCH * (888 + 444)));
     if (e != cudaSuccess) return e;
   }
   const dim3 grid((unsigned)((ntile + tiles - 1) / tiles), 3 * chunks, g.ns * PW);

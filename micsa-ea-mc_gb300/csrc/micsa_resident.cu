@@ -455,6 +455,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
 }
 
 /* ------------------------------------------------------------- launches */
+constexpr size_t STATIC_SMEM = 64; /* at least the kernel's mbarriers */
 using kern_t = void (*)(micsa_geo, slice, uint32_t *, uint32_t *, uint32_t *, const uint8_t *,
                         const int *);
 struct variant {
@@ -475,8 +476,8 @@ const variant *variants(int *n) {
   *n = (int)(sizeof v / sizeof v[0]);
   return v;
 }
-cudaError_t config(const variant &v, int nc, int W, int ns, cudaStream_t st,
-                   cudaLaunchAttribute *at, cudaLaunchConfig_t *c) {
+void config(const variant &v, int nc, int W, int ns, cudaStream_t st, cudaLaunchAttribute *at,
+            cudaLaunchConfig_t *c) {
   *c = {};
   c->gridDim = dim3((unsigned)v.C, (unsigned)W, (unsigned)ns);
   c->blockDim = dim3((unsigned)v.T);
@@ -487,8 +488,16 @@ cudaError_t config(const variant &v, int nc, int W, int ns, cudaStream_t st,
   at->val.clusterDim.y = at->val.clusterDim.z = 1;
   c->attrs = at;
   c->numAttrs = 1;
-  return cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)c->dynamicSmemBytes);
+}
+/* The limit of a kernel's dynamic shared memory belongs to the function, not to
+ * the launch or the context: it is raised to what the deepest context (nc = 6,
+ * or fewer where the device has less) may ask for, always to the same value,
+ * so that contexts of other threads never lower it between each other's
+ * launches. */
+cudaError_t raise_limit(const variant &v, int optin) {
+  int nc = 6;
+  while (nc > 1 && v.smem(nc) + STATIC_SMEM > (size_t)optin) nc--;
+  return cudaFuncSetAttribute(v.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem(nc));
 }
 
 } /* namespace */
@@ -515,11 +524,12 @@ cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pi
   int n;
   const variant *v = variants(&n);
   for (int i = 0; i < n; i++) {
-    if (v[i].L != L || v[i].smem(nc) + 64 > (size_t)optin || (pin > 0 && v[i].C != pin)) continue;
+    if (v[i].L != L || v[i].smem(nc) + STATIC_SMEM > (size_t)optin || (pin > 0 && v[i].C != pin)) continue;
     cudaLaunchAttribute at;
     cudaLaunchConfig_t c;
     int fit = 0;
-    cudaError_t e = config(v[i], nc, W, ns, 0, &at, &c);
+    config(v[i], nc, W, ns, 0, &at, &c);
+    cudaError_t e = raise_limit(v[i], optin);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&fit, v[i].k, &c);
     if (e != cudaSuccess) return e;
     if (fit < 1) continue;
@@ -564,7 +574,9 @@ cudaError_t micsa_launch_resident(const micsa_geo &g, int cluster, int at_once, 
     if (v[i].L != g.L || v[i].C != cluster) continue;
     cudaLaunchAttribute at;
     cudaLaunchConfig_t c;
-    cudaError_t e = R > 1 ? config(v[i], g.nc, M, 1, st, &at, &c) : config(v[i], g.nc, g.W, g.ns, st, &at, &c);
+    if (R > 1) config(v[i], g.nc, M, 1, st, &at, &c);
+    else config(v[i], g.nc, g.W, g.ns, st, &at, &c);
+    cudaError_t e = cudaSuccess;
     for (int first = 0; first < R * U && e == cudaSuccess; first += M) {
       /* exactly the places that are left: a test for them in the kernel cost
        * its half-sweeps 8% (L=32) */
