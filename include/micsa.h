@@ -432,7 +432,10 @@ int micsa_multi_report(const micsa_multi *m, char *buf, size_t n);
 int micsa_set_active(micsa_ctx *ctx, const uint8_t *active);
 
 /* Wait for all work issued on the context (cudaDeviceSynchronize,
- * main.cu:144,149) and report any asynchronous error. */
+ * main.cu:144,149) and report any asynchronous error.  A bounded wait of the
+ * cluster exchange (resident kernel, L = 16, 24, 32) that ran out is reported
+ * as MICSA_ERR_CUDA, once, by the context's next call that waits for its
+ * stream: this one, micsa_measure, a download, or micsa_multi_synchronize. */
 int micsa_synchronize(micsa_ctx *ctx);
 /* Test hook for the bounded device waits; no counterpart in the reference,
  * whose failed CUDA calls exit (cudamacro.h:1-16).  The dataflow sweep
@@ -444,7 +447,10 @@ int micsa_synchronize(micsa_ctx *ctx);
  * counters reach, so that every wait runs out: the iteration then completes
  * without its ordering and its results are not valid.  The setting holds
  * for every context on the device until changed; micsa_debug_flow_waits(ctx,
- * 0, 0) restores operation.  Synchronises the context's stream. */
+ * 0, 0) restores operation.  The same limit, in tries of about 2 us, and the
+ * same running out apply to the waits of this context's cluster exchange,
+ * whose report is the context's own (see micsa_synchronize).  Synchronises
+ * the context's stream. */
 int micsa_debug_flow_waits(micsa_ctx *ctx, uint64_t limit_ns, int unreachable);
 
 /* Number of kernels this context has launched so far (graph replays count

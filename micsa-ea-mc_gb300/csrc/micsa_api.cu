@@ -56,6 +56,8 @@ struct micsa_ctx {
                               this many blocks per sample and replica word (0: not) */
   int resident_once = 0;    /* of these clusters the GPU runs at once (0: not asked) */
   int64_t resident_min = 1; /* calls of fewer iterations run half-sweep by half-sweep */
+  micsa_waits waits = {nullptr, MICSA_WAIT_TRIES, 0}; /* of the cluster exchange */
+  unsigned *waits_out = nullptr; /* the host's view of their count */
   int split = 0;           /* k > 0: half-sweep launches per group of k samples, group-major
                               (a smaller L2 working set); 0: all samples per launch */
   int chains = 1;          /* an iteration's launches in the graph: chains of samples side by side */
@@ -196,6 +198,18 @@ uint64_t *device_view(const uint64_t *p, int64_t n) {
     at[k] = (char *)a.devicePointer;
   }
   return at[1] - at[0] == (const char *)ends[1] - (const char *)ends[0] ? (uint64_t *)at[0] : nullptr;
+}
+
+/* Whether waits of the context's cluster exchange have run out, its stream being
+ * idle: reported once, by the first call that waits for the stream (counted per
+ * context, so that no other context's call takes the report). */
+int check_waits(micsa_ctx *ctx) {
+  const unsigned n = ctx->waits_out ? *(volatile unsigned *)ctx->waits_out : 0u;
+  if (!n) return MICSA_OK;
+  *(volatile unsigned *)ctx->waits_out = 0;
+  return fail(ctx, MICSA_ERR_CUDA,
+              "%u waits of the cluster-resident sweep timed out: the results of that "
+              "iteration are not valid", n);
 }
 
 int ready_for_sweeps(micsa_ctx *ctx, int need_demons) {
@@ -964,6 +978,11 @@ int create_ctx(const micsa_config *cfg, bool shared, micsa_ctx **out) {
                                            &ctx->resident_once, &ctx->resident_min));
     /* beside other contexts' kernels a last wave leaves them its SMs */
     if (shared) ctx->resident_once = 0;
+    if (ctx->resident > 1) {
+      MICSA_CK_CREATE(cudaHostAlloc(&ctx->waits_out, sizeof(unsigned), cudaHostAllocMapped));
+      *ctx->waits_out = 0;
+      MICSA_CK_CREATE(cudaHostGetDevicePointer((void **)&ctx->waits.ran_out, ctx->waits_out, 0));
+    }
   }
   MICSA_CK_CREATE(micsa_make_tma(ctx->g, ctx->dem0, ctx->dem1, &ctx->tma));
   if ((rc = autotune(ctx)) != MICSA_OK) {
@@ -1035,6 +1054,7 @@ int micsa_destroy(micsa_ctx *ctx) {
   for (cudaEvent_t e : ctx->chain_ev)
     if (e) cudaEventDestroy(e);
   micsa_refresh_plan_free(&ctx->plan);
+  if (ctx->waits_out) cudaFreeHost(ctx->waits_out);
   if (ctx->rec_host) cudaFreeHost(ctx->rec_host);
   if (ctx->rec_copied) cudaEventDestroy(ctx->rec_copied);
   delete ctx;
@@ -1467,7 +1487,8 @@ int micsa_iterate(micsa_ctx *ctx, int64_t n) {
     for (int64_t done = 0; done < n;) {
       const int m = (int)(n - done < 1024 ? n - done : 1024);
       MICSA_CK(micsa_launch_resident(ctx->g, ctx->resident, ctx->resident_once, m, ctx->spin, ctx->dem0,
-                                     ctx->dem1, ctx->jb, ctx->walk, ctx->stream, &ctx->launches));
+                                     ctx->dem1, ctx->jb, ctx->walk, ctx->waits, ctx->stream,
+                                     &ctx->launches));
       done += m;
     }
     return MICSA_OK;
@@ -1501,6 +1522,7 @@ int micsa_measure(micsa_ctx *ctx, int32_t *e_spin, uint64_t *e_demon, int64_t *q
   std::vector<unsigned long long> h(ctx->acc_words);
   MICSA_CK(cudaMemcpyAsync(h.data(), ctx->acc, 8 * ctx->acc_words, cudaMemcpyDeviceToHost, ctx->stream));
   MICSA_CK(cudaStreamSynchronize(ctx->stream));
+  if ((rc = check_waits(ctx))) return rc;
   const int64_t V = 2 * g.P;
   const unsigned long long *hu = h.data(), *hd = hu + ns * nr, *hq = hd + ns * nr,
                            *hc = hq + ns * np;
@@ -1536,7 +1558,7 @@ int micsa_download_spins(micsa_ctx *ctx, int sample, uint64_t *even, uint64_t *o
     MICSA_CK(cudaMemcpyAsync(odd, ctx->stage + n, 8 * n, cudaMemcpyDeviceToHost, ctx->stream));
   }
   MICSA_CK(cudaStreamSynchronize(ctx->stream));
-  return MICSA_OK;
+  return check_waits(ctx);
 }
 
 int micsa_download_demons(micsa_ctx *ctx, int sample, uint64_t *w0, uint64_t *w1) {
@@ -1563,7 +1585,7 @@ int micsa_download_demons(micsa_ctx *ctx, int sample, uint64_t *w0, uint64_t *w1
     }
   }
   MICSA_CK(cudaStreamSynchronize(ctx->stream));
-  return MICSA_OK;
+  return check_waits(ctx);
 }
 
 int micsa_profile(micsa_ctx *ctx, int64_t n, double *sweep_ms, double *iteration_ms) {
@@ -1652,16 +1674,7 @@ int micsa_synchronize(micsa_ctx *ctx) {
                 "%u waits of the dataflow sweep timed out: the results of that iteration are "
                 "not valid", to);
   }
-  if (ctx->resident > 1) {
-    MICSA_CK(micsa_cluster_timeout_count(&to));
-    if (to) {
-      MICSA_CK(micsa_cluster_timeout_clear());
-      return fail(ctx, MICSA_ERR_CUDA,
-                  "%u waits of the cluster-resident sweep timed out: the results of that "
-                  "iteration are not valid", to);
-    }
-  }
-  return MICSA_OK;
+  return check_waits(ctx);
 }
 
 int micsa_debug_flow_waits(micsa_ctx *ctx, uint64_t limit_ns, int unreachable) {
@@ -1671,6 +1684,10 @@ int micsa_debug_flow_waits(micsa_ctx *ctx, uint64_t limit_ns, int unreachable) {
   MICSA_CK(cudaStreamSynchronize(ctx->stream));
   MICSA_CK(micsa_flow_set_waits(limit_ns ? (unsigned long long)limit_ns : 2000000000ull,
                                 unreachable ? 0x40000000u : 0u, ctx->stream));
+  /* a try that fails has taken 0.2 to 4 us (L = 16 to 32) */
+  const uint64_t tries = limit_ns / 2000 + 1;
+  ctx->waits.tries = limit_ns && tries < MICSA_WAIT_TRIES ? (int)tries : MICSA_WAIT_TRIES;
+  ctx->waits.withheld = unreachable ? 1 : 0;
   return MICSA_OK;
 }
 
@@ -2133,6 +2150,9 @@ int micsa_multi_synchronize(micsa_multi *m) {
     MULTI_CK(micsa_flow_timeout_clear());
     return mfail(m, MICSA_ERR_CUDA, "%u waits of the mixed dataflow sweep timed out", to);
   }
+  for (size_t gi = 0; gi < m->ctx.size(); gi++)
+    if (m->own[gi] && check_waits(m->ctx[gi]))
+      return mfail(m, MICSA_ERR_CUDA, "group %zu: %s", gi, m->ctx[gi]->err);
   return MICSA_OK;
 }
 

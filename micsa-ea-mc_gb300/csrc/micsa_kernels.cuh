@@ -198,19 +198,27 @@ cudaError_t micsa_launch_refresh(const micsa_geo &g, int first, int count, int64
                                  const uint64_t *fib, const uint64_t thr[3],
                                  uint32_t *dem0, uint32_t *dem1, cudaStream_t st);
 
+/* The bounded waits of the resident kernel's cluster exchange, of one context:
+ * where those that ran out are counted (a mapped host word), after how many
+ * tries of the mbarrier one gives up, and, for a test, 1 to let every wait run
+ * out (its mbarriers are initialised with an arrival that never comes). */
+#define MICSA_WAIT_TRIES (1 << 20)
+struct micsa_waits {
+  unsigned *ran_out;
+  int tries;
+  int withheld;
+};
+
 /* The cluster size (blocks per sample and replica word) with which the
  * resident kernel runs this shape, pin > 0 asking for that size; 0: not a
  * shape it holds; how many clusters run at once (0 when pinned); and the
  * iterations from which it pays.  Its launches: n whole iterations of all
  * samples, walk counters advanced by n; with at_once > 0, where that saves a
- * mostly idle last wave, in rounds over several launches.  Waits of its
- * cluster exchange that ran out. */
+ * mostly idle last wave, in rounds over several launches. */
 cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pin, int *cluster,
                                  int *at_once, int64_t *min_n);
 cudaError_t micsa_launch_resident(const micsa_geo &g, int cluster, int at_once, int n, uint32_t *spin,
                                   uint32_t *d0, uint32_t *d1, const uint8_t *jb, int *walk,
-                                  cudaStream_t st, int64_t *launches);
-cudaError_t micsa_cluster_timeout_count(unsigned *n);
-cudaError_t micsa_cluster_timeout_clear();
+                                  const micsa_waits &wt, cudaStream_t st, int64_t *launches);
 
 #endif

@@ -41,21 +41,37 @@ __device__ __forceinline__ uint2 word_pair(const uint32_t *a, int W, int w) {
   if (W == 1) return *(const uint2 *)a;
   return make_uint2(a[w], a[W + w]);
 }
-/* Waits of the cluster exchange that ran out (a peer that never pushed).
- * After one, every later wait gives up at once: the launch ends and
- * micsa_synchronize reports it. */
-__device__ unsigned int micsa_cluster_timeouts;
-__device__ __forceinline__ void halo_wait(uint64_t *bar, uint32_t phase) {
-  const uint32_t a = smem_addr(bar);
-  for (int i = 0; i < (1 << 20); i++) {
-    uint32_t done;
-    asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2; "
-                 "selp.u32 %0, 1, 0, q; }"
-                 : "=r"(done) : "r"(a), "r"(phase) : "memory");
-    if (done) return;
-    if ((i & 1023) == 1023 && *(volatile unsigned *)&micsa_cluster_timeouts) return;
+__device__ __forceinline__ bool try_phase(uint32_t bar, uint32_t phase) {
+  uint32_t done;
+  asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2; "
+               "selp.u32 %0, 1, 0, q; }"
+               : "=r"(done) : "r"(bar), "r"(phase) : "memory");
+  return done;
+}
+/* Waits of the cluster exchange: one try in line, the others here (all of them
+ * in line in the half-sweep's code cost L=16 12% and L=32 4% of their time).
+ * Bounded by tries, which count only while the cluster runs; once a wait of the
+ * context has run out the others give up at their 1024th.
+ *
+ * A thread whose wait ran out (a peer that never pushed) counts it in the
+ * context's word, which the host looks at whenever it has waited for the stream,
+ * and ends: barriers wait for the threads that are left, nothing is pushed or
+ * re-armed on the strength of words that did not come, and the threads that
+ * depend on its own words run out in turn.  It ends late, by a millisecond or
+ * so, since a block's shared memory must outlast the pushes to it: a neighbour
+ * issues its last ones within an iteration (10 us) of the first word it misses. */
+__device__ __noinline__ void halo_wait_more(uint32_t bar, uint32_t phase, unsigned *ran_out, int tries) {
+  for (int i = 0; i < tries; i++) {
+    if (try_phase(bar, phase)) return;
+    if ((i & 1023) == 1023 && *(volatile unsigned *)ran_out) break;
   }
-  atomicAdd(&micsa_cluster_timeouts, 1u);
+  atomicAdd_system(ran_out, 1u);
+  for (int i = 0; i < 1000; i++) __nanosleep(2000);
+  asm volatile("exit;");
+}
+__device__ __forceinline__ void halo_wait(uint64_t *bar, uint32_t phase, const micsa_waits &wt) {
+  const uint32_t a = smem_addr(bar);
+  if (!try_phase(a, phase)) halo_wait_more(a, phase, wt.ran_out, wt.tries);
 }
 
 /* ---------------------------------------------------------------- shape */
@@ -133,7 +149,7 @@ struct slice {
  * waits for them an iteration later.  The last iteration keeps its demons and
  * the final copy stores them at their place.
  *
- * Waits are bounded; see halo_wait.
+ * Waits are bounded; see halo_wait_more.
  *
  * What bounds it: with one block per sample the integer ALU pipe (75% busy at
  * L=16, 58 of 86 instructions per pair and half-sweep; 1.2 us of the 15 ...
@@ -153,7 +169,7 @@ template <int L, int C, int PPT>
 __global__ void __launch_bounds__((rcfg<L, C, PPT>::T), 1)
 k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
            uint32_t *__restrict__ d0, uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb,
-           const int *__restrict__ walk) {
+           const int *__restrict__ walk, const micsa_waits wt) {
   using K = rcfg<L, C, PPT>;
   constexpr int Lh = K::Lh, R = K::R, PL = K::PL, Zc = K::Zc, NPP = K::NPP, T = K::T, KZ = K::KZ,
                 HZ = K::HZ, P = L * PL;
@@ -254,7 +270,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
     }
   constexpr uint32_t HALO_BYTES = 2 * PB, DEM_BYTES = 4 * PB;
   if (CL && tid == 0) {
-    for (int b = 0; b < 6; b++) mbar_init(bars + b, 1);
+    for (int b = 0; b < 6; b++) mbar_init(bars + b, 1 + wt.withheld);
     mbar_fence_init();
     for (int b = 0; b < 2; b++) mbar_expect_tx(bars + b, HALO_BYTES);
     for (int b = 2; b < 6; b++) mbar_expect_tx(bars + b, DEM_BYTES);
@@ -312,7 +328,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
         }
         if (zx && it > 0) { /* the planes that entered since the last iteration */
           uint64_t *b = bars + 2 + (ic == 5 ? 2 : 0) + p;
-          halo_wait(b, (uint32_t)(it - 1) & 1);
+          halo_wait(b, (uint32_t)(it - 1) & 1, wt);
           if (tid == 0) mbar_expect_tx(b, DEM_BYTES);
         }
         int xd = j2 - shx, yd = y - shy;
@@ -342,7 +358,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
 #pragma unroll
         for (int k = 0; k < PPT; k++) {
           if (CL && k == PPT - 1 && jn > 0 && (low || high)) {
-            halo_wait(bars + q, ((jn - 1) >> 1) & 1);
+            halo_wait(bars + q, ((jn - 1) >> 1) & 1, wt);
             if (tid == 0) mbar_expect_tx(bars + q, HALO_BYTES);
           }
           constexpr uint32_t oq = q * HZ * PB;
@@ -417,7 +433,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
 
   /* the last half-sweep's words must have arrived before this block ends */
   if (CL) {
-    halo_wait(bars + 1, ((jn - 1) >> 1) & 1);
+    halo_wait(bars + 1, ((jn - 1) >> 1) & 1, wt);
     cluster_sync();
   }
 #pragma unroll 4
@@ -457,7 +473,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
 /* ------------------------------------------------------------- launches */
 constexpr size_t STATIC_SMEM = 64; /* at least the kernel's mbarriers */
 using kern_t = void (*)(micsa_geo, slice, uint32_t *, uint32_t *, uint32_t *, const uint8_t *,
-                        const int *);
+                        const int *, micsa_waits);
 struct variant {
   int L, C, T;
   size_t (*smem)(int);
@@ -566,7 +582,7 @@ static int resident_rounds(int64_t U, int64_t M, int n) {
 
 cudaError_t micsa_launch_resident(const micsa_geo &g, int cluster, int at_once, int n, uint32_t *spin,
                                   uint32_t *d0, uint32_t *d1, const uint8_t *jb, int *walk,
-                                  cudaStream_t st, int64_t *launches) {
+                                  const micsa_waits &wt, cudaStream_t st, int64_t *launches) {
   int nv;
   const variant *v = variants(&nv);
   const int U = g.W * g.ns, R = resident_rounds(U, at_once, n), M = R > 1 ? at_once : U;
@@ -581,7 +597,8 @@ cudaError_t micsa_launch_resident(const micsa_geo &g, int cluster, int at_once, 
       /* exactly the places that are left: a test for them in the kernel cost
        * its half-sweeps 8% (L=32) */
       if (R > 1) c.gridDim.y = (unsigned)(R * U - first < M ? R * U - first : M);
-      e = cudaLaunchKernelEx(&c, v[i].k, g, slice{n, R, U, first}, spin, d0, d1, jb, (const int *)walk);
+      e = cudaLaunchKernelEx(&c, v[i].k, g, slice{n, R, U, first}, spin, d0, d1, jb, (const int *)walk,
+                             wt);
       ++*launches;
     }
     if (e != cudaSuccess) return e;
@@ -589,12 +606,4 @@ cudaError_t micsa_launch_resident(const micsa_geo &g, int cluster, int at_once, 
     return micsa_launch_walk_add(g, walk, n, st);
   }
   return cudaErrorInvalidValue;
-}
-
-cudaError_t micsa_cluster_timeout_count(unsigned *n) {
-  return cudaMemcpyFromSymbol(n, micsa_cluster_timeouts, sizeof(unsigned));
-}
-cudaError_t micsa_cluster_timeout_clear() {
-  const unsigned zero = 0;
-  return cudaMemcpyToSymbol(micsa_cluster_timeouts, &zero, sizeof(unsigned));
 }
