@@ -409,11 +409,12 @@ int autotune(micsa_ctx *ctx) {
       if (g.flow && k >= 1 && k <= 64) g.fit = k;
     }
     if (const char *eh = getenv("MICSA_SWEEP_CHAINS")) {
-      /* K or K/U: chains, iterations per graph replay */
+      /* K or K/U: chains, iterations per graph replay; 1/1 with a sample order of
+       * its own (MICSA_SWEEP_SPLIT), whose launches are one iteration's */
       int K = atoi(eh), U = strchr(eh, '/') ? atoi(strchr(eh, '/') + 1) : 1;
       K = K < 1 ? 1 : (K > MICSA_CHAINS_MAX ? MICSA_CHAINS_MAX : K);
       ctx->chains = g.flow || ctx->split ? 1 : (K < g.ns ? K : g.ns);
-      ctx->unit = g.flow || U < 1 ? 1 : (U > 64 ? 64 : U);
+      ctx->unit = g.flow || ctx->split || U < 1 ? 1 : (U > 64 ? 64 : U);
       MICSA_CK(ensure_chains(ctx, ctx->chains));
     }
     const int oc = eo ? atoi(eo) : 3;
