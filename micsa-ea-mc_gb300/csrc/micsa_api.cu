@@ -706,7 +706,16 @@ int autotune(micsa_ctx *ctx) {
    * samples x 32 replicas: 218 -> 174 us per iteration; L=48, 32 x 64: 193 ->
    * 158; L=128, 2 x 64: 160 against 176 for the dataflow sweep), four and
    * several iterations per replay help the smallest launches (L=48, 4 x 64:
-   * 43.6 -> 38.9 with two chains and four iterations). */
+   * 43.6 -> 38.9 with two chains and four iterations).
+   *
+   * The contexts of a batch's groups and a server's pools fill each other's
+   * drains, and the GPU starts about one launch per microsecond for all of
+   * them: theirs are cut into chains only while a chain's launch lasts 4 us or
+   * more.  us per iteration and context, four side by side, chains freely and
+   * by this rule: L=24, 60 x 64 55 and 37; L=64, 4 x 64 49 and 42; L=96, 4 x 64
+   * 171 and 184 (K=4 and 2).  The bench's streams, anneals/s: batched 91 to 92
+   * freely, 97 by the rule, 89 without chains; served (60 requests) 6.0, 6.5
+   * and 5.5, (200 requests) 5.7, 5.9 and 6.2. */
   {
     double base = 1e30; /* ms per iteration of the choice so far */
     if (g.flow) base = best_flow_it;
@@ -768,6 +777,7 @@ int autotune(micsa_ctx *ctx) {
           g.tw = ctx->tune_tw[c];
           double per = 0;
           if ((rc = time_chains(K, U, &per))) return rc;
+          if (ctx->shared && K > 1 && per < 4e-3 * K * 2 * g.nc) continue;
           if (per < base) {
             base = per;
             pick = g;
