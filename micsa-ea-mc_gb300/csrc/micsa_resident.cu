@@ -48,10 +48,9 @@ __device__ __forceinline__ bool try_phase(uint32_t bar, uint32_t phase) {
                : "=r"(done) : "r"(bar), "r"(phase) : "memory");
   return done;
 }
-/* Waits of the cluster exchange: one try in line, the others here (all of them
- * in line in the half-sweep's code cost L=16 12% and L=32 4% of their time).
- * Bounded by tries, which count only while the cluster runs; once a wait of the
- * context has run out the others give up at their 1024th.
+/* Waits of the cluster exchange.  Bounded by tries, which count only while the
+ * cluster runs; once a wait of the context has run out the others give up at
+ * their 1024th.
  *
  * A thread whose wait ran out (a peer that never pushed) counts it in the
  * context's word, which the host looks at whenever it has waited for the stream,
@@ -60,18 +59,30 @@ __device__ __forceinline__ bool try_phase(uint32_t bar, uint32_t phase) {
  * depend on its own words run out in turn.  It ends late, by a millisecond or
  * so, since a block's shared memory must outlast the pushes to it: a neighbour
  * issues its last ones within an iteration (10 us) of the first word it misses. */
-__device__ __noinline__ void halo_wait_more(uint32_t bar, uint32_t phase, unsigned *ran_out, int tries) {
-  for (int i = 0; i < tries; i++) {
-    if (try_phase(bar, phase)) return;
-    if ((i & 1023) == 1023 && *(volatile unsigned *)ran_out) break;
-  }
+__device__ __noinline__ void halo_lost(unsigned *ran_out) {
   atomicAdd_system(ran_out, 1u);
   for (int i = 0; i < 1000; i++) __nanosleep(2000);
   asm volatile("exit;");
 }
-__device__ __forceinline__ void halo_wait(uint64_t *bar, uint32_t phase, const micsa_waits &wt) {
+__device__ __forceinline__ void halo_tries(uint32_t bar, uint32_t phase, const micsa_waits *wt) {
+  for (int i = 0;; i++) {
+    if (try_phase(bar, phase)) return;
+    if ((i & 1023) == 1023 && (i >= wt->tries || *(volatile unsigned *)wt->ran_out)) break;
+  }
+  halo_lost(wt->ran_out);
+}
+__device__ __noinline__ void halo_tries_call(uint32_t bar, uint32_t phase, const micsa_waits *wt) {
+  halo_tries(bar, phase, wt);
+}
+/* CALL: one try in line, the others out of it, which shortens the half-sweep's
+ * code: us per iteration, all tries in line and so, L=16 x 1 by 8 blocks 3.02 and
+ * 2.88, by 4 4.01 and 3.97, L=32 x 2 9.77 and 9.56.  Where the threads next to a
+ * neighbour do not fill their warps and hold two pairs, the call costs more than
+ * it saves: L=24 x 2 by 4 blocks 8.68 and 9.55. */
+template <bool CALL> __device__ __forceinline__ void halo_wait(uint64_t *bar, uint32_t phase, const micsa_waits *wt) {
   const uint32_t a = smem_addr(bar);
-  if (!try_phase(a, phase)) halo_wait_more(a, phase, wt.ran_out, wt.tries);
+  if (!CALL) halo_tries(a, phase, wt);
+  else if (!try_phase(a, phase)) halo_tries_call(a, phase, wt);
 }
 
 /* ---------------------------------------------------------------- shape */
@@ -88,6 +99,7 @@ template <int L, int C, int PPT> struct rcfg {
   static constexpr int Zc = L / C, NPP = L * R;             /* planes, pairs per plane */
   static constexpr int T = Zc * NPP / PPT, KZ = Zc / PPT;
   static constexpr int HZ = C > 1 ? Zc + 2 : Zc; /* spin planes with their halos */
+  static constexpr bool CALL = PPT == 1 || NPP % 32 == 0; /* see halo_wait */
   static_assert(L % C == 0 && Zc >= 2 && Zc % PPT == 0 && PPT <= 2 && T <= 1024, "shape");
   /* at most one pair of a thread leaves along z, an inner plane is no edge */
   static_assert(C == 1 || PPT == 1 || KZ >= 2, "shape");
@@ -149,7 +161,7 @@ struct slice {
  * waits for them an iteration later.  The last iteration keeps its demons and
  * the final copy stores them at their place.
  *
- * Waits are bounded; see halo_wait_more.
+ * Waits are bounded; see halo_lost.
  *
  * What bounds it: with one block per sample the integer ALU pipe (75% busy at
  * L=16, 58 of 86 instructions per pair and half-sweep; 1.2 us of the 15 ...
@@ -169,7 +181,7 @@ template <int L, int C, int PPT>
 __global__ void __launch_bounds__((rcfg<L, C, PPT>::T), 1)
 k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
            uint32_t *__restrict__ d0, uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb,
-           const int *__restrict__ walk, const micsa_waits wt) {
+           const int *__restrict__ walk, const __grid_constant__ micsa_waits wt) {
   using K = rcfg<L, C, PPT>;
   constexpr int Lh = K::Lh, R = K::R, PL = K::PL, Zc = K::Zc, NPP = K::NPP, T = K::T, KZ = K::KZ,
                 HZ = K::HZ, P = L * PL;
@@ -328,7 +340,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
         }
         if (zx && it > 0) { /* the planes that entered since the last iteration */
           uint64_t *b = bars + 2 + (ic == 5 ? 2 : 0) + p;
-          halo_wait(b, (uint32_t)(it - 1) & 1, wt);
+          halo_wait<K::CALL>(b, (uint32_t)(it - 1) & 1, &wt);
           if (tid == 0) mbar_expect_tx(b, DEM_BYTES);
         }
         int xd = j2 - shx, yd = y - shy;
@@ -358,7 +370,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
 #pragma unroll
         for (int k = 0; k < PPT; k++) {
           if (CL && k == PPT - 1 && jn > 0 && (low || high)) {
-            halo_wait(bars + q, ((jn - 1) >> 1) & 1, wt);
+            halo_wait<K::CALL>(bars + q, ((jn - 1) >> 1) & 1, &wt);
             if (tid == 0) mbar_expect_tx(bars + q, HALO_BYTES);
           }
           constexpr uint32_t oq = q * HZ * PB;
@@ -433,7 +445,7 @@ k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
 
   /* the last half-sweep's words must have arrived before this block ends */
   if (CL) {
-    halo_wait(bars + 1, ((jn - 1) >> 1) & 1, wt);
+    halo_wait<K::CALL>(bars + 1, ((jn - 1) >> 1) & 1, &wt);
     cluster_sync();
   }
 #pragma unroll 4
