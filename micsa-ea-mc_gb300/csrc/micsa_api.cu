@@ -985,7 +985,7 @@ int create_ctx(const micsa_config *cfg, bool shared, micsa_ctx **out) {
                                            cfg->device));
     if (!(er && !strcmp(er, "0")) && (cfg->L <= 16 || !getenv("MICSA_SWEEP_ZC")))
       MICSA_CK_CREATE(micsa_resident_shape(cfg->L, cfg->nc, g.W, cfg->nsamples, optin,
-                                           ec ? atoi(ec) : 0, &ctx->resident,
+                                           ec ? atoi(ec) : 0, shared, &ctx->resident,
                                            &ctx->resident_once, &ctx->resident_min));
     /* beside other contexts' kernels a last wave leaves them its SMs */
     if (shared) ctx->resident_once = 0;

@@ -212,11 +212,11 @@ struct micsa_waits {
 /* The cluster size (blocks per sample and replica word) with which the
  * resident kernel runs this shape, pin > 0 asking for that size; 0: not a
  * shape it holds; how many clusters run at once (0 when pinned); and the
- * iterations from which it pays.  Its launches: n whole iterations of all
+ * iterations from which it pays, alone or beside other contexts' kernels.  Its launches: n whole iterations of all
  * samples, walk counters advanced by n; with at_once > 0, where that saves a
  * mostly idle last wave, in rounds over several launches. */
-cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pin, int *cluster,
-                                 int *at_once, int64_t *min_n);
+cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pin, bool beside,
+                                 int *cluster, int *at_once, int64_t *min_n);
 cudaError_t micsa_launch_resident(const micsa_geo &g, int cluster, int at_once, int n, uint32_t *spin,
                                   uint32_t *d0, uint32_t *d1, const uint8_t *jb, int *walk,
                                   const micsa_waits &wt, cudaStream_t st, int64_t *launches);

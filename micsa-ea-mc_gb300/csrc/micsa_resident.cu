@@ -540,12 +540,22 @@ cudaError_t raise_limit(const variant &v, int optin) {
  * *min_n: the least number of iterations in a call that pays for copying the
  * state in and out.  A launch of v waves of clusters costs about v times
  * (15 to 35 us + its iterations), the half-sweep launches 23 to 115 us per
- * iteration; measured, they meet at n = v or just above it: one wave at
- * L <= 24 wins from n = 1 (L=24 x 2: 22 against 24 us), at L = 32 from n = 2
- * (48 against 62; n = 1: 38 against 31), four waves (L=32 x 24 samples) from
- * n = 5 (n = 4: 245 against 243 us, n = 8: 399 against 486). */
-cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pin, int *cluster,
-                                 int *at_once, int64_t *min_n) {
+ * iteration; measured, they meet at n = v or just above it for L = 24 and 32:
+ * one wave at L = 24 wins from n = 1 (L=24 x 2: 22 against 24 us), at L = 32
+ * from n = 2 (48 against 62; n = 1: 38 against 31), four waves (L=32 x 24
+ * samples) from n = 5 (n = 4: 245 against 243 us, n = 8: 399 against 486).  At
+ * L <= 16 n = 2 pays for any number of waves (L=16 x 100 samples, two waves: 83
+ * against 91 us; x 300, four: 175 against 187; n = 1: 97 by half-sweeps).
+ *
+ * `beside`: contexts at work side by side fill the gaps of each other's
+ * half-sweep launches, not of launches that hold whole SMs.  us per call, three
+ * contexts, resident and half-sweeps: L=32 x 24 samples (four waves) n = 8 321
+ * and 288, 12 441 and 433, 16 562 and 577; L=32 x 10 (two) 4 82 and 79, 6 107 and
+ * 118; L=32 x 60 (eight) 12 1099 and 920, 24 2000 and 1830; L=24 x 60 (four) 8 316
+ * and 313, 11 402 and 430; L=16 x 300 (four) 3 194 and 215, 4 222 and 295, 2 166
+ * and 146. */
+cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pin, bool beside,
+                                 int *cluster, int *at_once, int64_t *min_n) {
   *cluster = 0;
   *at_once = 0;
   *min_n = 1;
@@ -565,7 +575,10 @@ cudaError_t micsa_resident_shape(int L, int nc, int W, int ns, int optin, int pi
     if (*cluster == 0 || waves == 1) {
       *cluster = v[i].C;
       *at_once = pin > 0 ? 0 : fit;
-      *min_n = pin > 0 ? 1 : waves + (waves > 1 || L > 24);
+      if (pin > 0) *min_n = 1;
+      else if (waves == 1) *min_n = 1 + (L > 24);
+      else if (L <= 16) *min_n = beside && waves > 2 ? 3 : 2;
+      else *min_n = beside ? (L > 24 ? 3 : 2) * waves : waves + 1;
     }
   }
   return cudaSuccess;

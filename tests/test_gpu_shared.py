@@ -50,3 +50,28 @@ def test_side_by_side_no_chains_of_short_launches(monkeypatch):
             c.iterate(3)
         for x, y in zip(a.download_spins(0) + a.download_demons(0), b.download_spins(0) + b.download_demons(0)):
             assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("L,ns,shared,halves,resident", [
+    (16, 100, False, 1, 2), (16, 300, False, 1, 2), (16, 300, True, 2, 3),  # two and four waves of clusters
+    (32, 24, False, 4, 5), (32, 24, True, 11, 12), (24, 4, True, 0, 1)])
+def test_calls_long_enough_to_run_in_shared_memory(monkeypatch, L, ns, shared, halves, resident):
+    """calls of up to `halves` iterations run half-sweep by half-sweep, of `resident` and more in
+    one or a few launches; the same state either way"""
+    monkeypatch.setenv("MICSA_SWEEP_FLOW", "0")
+    J, e, o, w0, w1, _ = random_state(np.random.default_rng(L), L, 64, 6, 1)[0]
+    with _context(L, 64, ns, 6, shared) as a, _context(L, 64, ns, 6, not shared) as b:
+        for c in (a, b):
+            c.set_active([0] * (ns - 1) + [1])
+            c.upload_couplings(ns - 1, J)
+            c.upload_spins(ns - 1, e, o)
+            c.upload_demons(ns - 1, w0, w1)
+        for n, whole in ((halves, False), (resident, True)):
+            before = a.kernel_launches()
+            if n:
+                a.iterate(n)
+                assert (a.kernel_launches() - before < 12) == whole, (n, a.kernel_launches() - before)
+                b.iterate(n)
+        for x, y in zip(a.download_spins(ns - 1) + a.download_demons(ns - 1),
+                        b.download_spins(ns - 1) + b.download_demons(ns - 1)):
+            assert np.array_equal(x, y)
