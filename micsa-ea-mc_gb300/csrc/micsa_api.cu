@@ -1469,7 +1469,9 @@ int micsa_monte_carlo(micsa_ctx *ctx, int flag, const uint32_t *te, const uint32
   return MICSA_OK;
 }
 
-int micsa_iterate(micsa_ctx *ctx, int64_t n) {
+/* micsa_iterate; beside: other contexts' kernels run at the same time, to which a
+ * small lattice's last wave of clusters leaves its SMs (no rounds) */
+static int iterate_ctx(micsa_ctx *ctx, int64_t n, bool beside) {
   if (!ctx || n < 0) return fail(ctx, MICSA_ERR_ARG, "bad argument");
   int rc = set_device(ctx);
   if (rc || (rc = ready_for_sweeps(ctx, 1))) return rc;
@@ -1497,8 +1499,8 @@ int micsa_iterate(micsa_ctx *ctx, int64_t n) {
     /* small lattices: whole iterations in shared memory, up to 1024 per launch */
     for (int64_t done = 0; done < n;) {
       const int m = (int)(n - done < 1024 ? n - done : 1024);
-      MICSA_CK(micsa_launch_resident(ctx->g, ctx->resident, ctx->resident_once, m, ctx->spin, ctx->dem0,
-                                     ctx->dem1, ctx->jb, ctx->walk, ctx->waits, ctx->stream,
+      MICSA_CK(micsa_launch_resident(ctx->g, ctx->resident, beside ? 0 : ctx->resident_once, m, ctx->spin,
+                                     ctx->dem0, ctx->dem1, ctx->jb, ctx->walk, ctx->waits, ctx->stream,
                                      &ctx->launches));
       done += m;
     }
@@ -1512,6 +1514,8 @@ int micsa_iterate(micsa_ctx *ctx, int64_t n) {
   }
   return MICSA_OK;
 }
+
+int micsa_iterate(micsa_ctx *ctx, int64_t n) { return iterate_ctx(ctx, n, false); }
 
 int micsa_measure(micsa_ctx *ctx, int32_t *e_spin, uint64_t *e_demon, int64_t *q, int64_t *c4) {
   if (!ctx) return MICSA_ERR_ARG;
@@ -2109,17 +2113,20 @@ int micsa_multi_iterate(micsa_multi *m, int64_t n) {
     if (ready_for_sweeps(c, 1)) return mfail(m, MICSA_ERR_STATE, "group %zu: %s", gi, c->err);
   }
   if (n == 0) return MICSA_OK;
+  const std::vector<unsigned> ns = multi_running(m);
+  bool any = false;
+  for (unsigned v : ns) any |= v > 0;
+  /* us per iteration, resident groups beside a launch in one launch a call and in
+   * rounds: L = 24, 32 and 48 with 20 samples each, 64 iterations 163 and 175;
+   * without a launch, L = 24 and 32 with 8, 256 iterations, 18.9 and 17.7 */
   for (size_t gi = 0; gi < m->ctx.size(); gi++)
     if (m->own[gi]) {
       micsa_ctx *c = m->ctx[gi];
       bool on = false;
       for (uint8_t v : c->active_host) on |= v != 0;
-      if (on && micsa_iterate(c, n))
+      if (on && iterate_ctx(c, n, any))
         return mfail(m, MICSA_ERR_CUDA, "group %zu: %s", gi, c->err);
     }
-  const std::vector<unsigned> ns = multi_running(m);
-  bool any = false;
-  for (unsigned v : ns) any |= v > 0;
   if (!any) return MICSA_OK;
   if (!m->exec || ns != m->graph_ns) {
     const int rc = multi_capture(m, ns);

@@ -75,3 +75,31 @@ def test_calls_long_enough_to_run_in_shared_memory(monkeypatch, L, ns, shared, h
         for x, y in zip(a.download_spins(ns - 1) + a.download_demons(ns - 1),
                         b.download_spins(ns - 1) + b.download_demons(ns - 1)):
             assert np.array_equal(x, y)
+
+
+def test_resident_groups_beside_a_mixed_launch_run_in_one_launch_a_call():
+    """20 clusters of L = 32 where about 15 run at once: in rounds when the context runs alone,
+    in one launch (and the walk's) while the mixed launch of the other context has work"""
+    shapes = [(32, 64, 10, 6), (48, 64, 1, 6)]
+    ctxs = [micsa.Context(*s) for s in shapes]
+    ref = micsa.Context(*shapes[0])
+    st = [random_state(np.random.default_rng(L), L, nr, nc, 1)[0] for L, nr, _, nc in shapes]
+    for c, (L, nr, ns, nc), (J, e, o, w0, w1, _) in zip(ctxs + [ref], shapes + shapes[:1], st + st[:1]):
+        for s in range(ns):
+            c.upload_couplings(s, J)
+            c.upload_spins(s, e, o)
+            c.upload_demons(s, w0, w1)
+    before = ref.kernel_launches()
+    ref.iterate(20)
+    assert ref.kernel_launches() - before > 2
+    with micsa.Multi(ctxs) as multi:
+        before = ctxs[0].kernel_launches()
+        multi.iterate(20)
+        assert ctxs[0].kernel_launches() - before == 2
+        multi.synchronize()
+    for s in (0, 9):
+        for x, y in zip(ctxs[0].download_spins(s) + ctxs[0].download_demons(s),
+                        ref.download_spins(s) + ref.download_demons(s)):
+            assert np.array_equal(x, y), s
+    for c in ctxs + [ref]:
+        c.close()
