@@ -344,7 +344,7 @@ cudaError_t ensure_chains(micsa_ctx *ctx, int K) {
  * choice and table instead of timing again, so batches and servers that open
  * many contexts of a few shapes pay for each shape once. */
 struct tune_entry {
-  int zc, pd, split, occ, tma, async, pipe, tw, flow, quad, fit, pers, half, xs, chains, unit, n;
+  int zc, pd, split, occ, tma, async, pipe, tw, flow, quad, fit, chains, unit, n; /* persistent, half-height, x-shuffle forms: pinned only */
   std::vector<int> zcs, pds, splits, occs, loads, tws;
   std::vector<double> ms;
 };
@@ -440,9 +440,6 @@ int autotune(micsa_ctx *ctx) {
       g.flow = t.flow;
       g.quad = t.quad;
       g.fit = t.fit;
-      g.pers = t.pers;
-      g.half = t.half;
-      g.xs = t.xs;
       ctx->chains = t.chains;
       ctx->unit = t.unit;
       MICSA_CK(ensure_chains(ctx, ctx->chains));
@@ -806,9 +803,6 @@ int autotune(micsa_ctx *ctx) {
     t.flow = g.flow;
     t.quad = g.quad;
     t.fit = g.fit;
-    t.pers = g.pers;
-    t.half = g.half;
-    t.xs = g.xs;
     t.chains = ctx->chains;
     t.unit = ctx->unit;
     t.n = n;
@@ -916,8 +910,9 @@ int create_ctx(const micsa_config *cfg, bool shared, micsa_ctx **out) {
   g.half = 0;
   g.xs = 0;
   {
-    /* MICSA_SWEEP_PF=n: the dataflow sweep requests n demon planes of each
-     * tile into L2 before its dependency wait (0: none) */
+    /* MICSA_SWEEP_PF=n: the dataflow sweep's block-shaped tiles (a pinned shape
+     * other than lin) request n demon planes each into L2 before their
+     * dependency wait (0: none) */
     const char *e = getenv("MICSA_SWEEP_PF");
     g.pf = e ? atoi(e) : 0;
     if (g.pf < 0) g.pf = 0;

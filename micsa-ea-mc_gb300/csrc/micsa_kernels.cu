@@ -671,8 +671,7 @@ k_sweep(const micsa_geo g, const int p, const int ic, const int ytiles, const in
         uint32_t *__restrict__ d1, const uint8_t *__restrict__ jb,
         const int *__restrict__ walk, const uint32_t *__restrict__ rnd,
         const __grid_constant__ micsa_tma tm) {
-  if (!MICSA) grid_launch_dependents(); /* the next colour's bits are drawn beside this sweep */
-  grid_dependency_sync();
+  grid_dependency_sync(); /* Metropolis: the next colour's bits are drawn beside this sweep */
   const uint32_t by = blockIdx.y;
   const uint32_t tile = by % ytiles, sg = by / ytiles; /* block-uniform */
   const uint32_t s = sg / G, grp = sg % G;
@@ -683,6 +682,7 @@ k_sweep(const micsa_geo g, const int p, const int ic, const int ytiles, const in
                                               zc, pd, kwalk, spin, d0, d1, jb, rnd, tm);
 }
 
+/* operands of one z step of a thread's S sites */
 template <int VW, int S> struct step_ops {
   uint32_t own[S * VW], up[S * VW], vn[S * VW], vs[S * VW], a0[S * VW], a1[S * VW], ext[VW];
   uint32_t jbs;
@@ -886,19 +886,22 @@ __device__ __forceinline__ void sweep_ahead_block(
  * only more than k slabs away, and reads one plane beyond its slab).  The
  * demon walk moves by whole iterations, between launches.
  *
- * Counters: ctl[0] tickets, ctl[1] blocks done, ctl[4 + s*nslab + b] tiles
- * of slab b of sample s finished in this launch.  No tile of j starts on
+ * Counters: ctl[0] tickets, ctl[4 + s*nslab + b] tiles of slab b of sample s
+ * finished in this launch (ctl[1]: blocks done, of the persistent form and the
+ * mixed launch).  No tile of j starts on
  * slab b before all of slab b's tiles of j-1 are done, so slab b has
  * finished half-sweeps 0 .. j-1 exactly when its counter reaches (tiles per
  * slab) * j.  Tiles wait only on earlier tickets, and a ticket is only held
  * by a running block, so the earliest unfinished tile can always run: the
- * launch needs no co-residency.  The lead thread polls the three counters
- * (first warp) polls the three counters with acquire loads, one lane each,
- * and a block barrier orders the tile's loads after the producers' stores; a
- * producer releases with the last of its warps' additions.  Waits are
- * bounded (2 s by the global timer; after one runs out every later wait
- * gives up at once, and micsa_flow_timeouts counts them); the last block to
- * finish resets the counters for the next launch. */
+ * launch needs no co-residency.  A block's first warp polls the three counters
+ * with acquire loads, one lane each, and a block barrier orders the tile's
+ * loads after the producers' stores; a producer's last warp to finish adds to
+ * its slab's counter with a release (the persistent form and the mixed launch
+ * poll and add by their lead thread).  Waits are bounded (2 s by the global
+ * timer; after one runs out every later wait gives up at once, and
+ * micsa_flow_timeouts counts them).  A memset after the launch clears the
+ * counters for the next one; in the persistent form and the mixed launch the
+ * last block to finish does. */
 __device__ unsigned int micsa_flow_timeouts;
 /* The wait limit, and an offset added to every wait's target count: 0 in
  * operation; set through micsa_debug_flow_waits so that a test can make the
@@ -1570,7 +1573,6 @@ k_sweep_async(const micsa_geo g, const int p, const int ic, const int ytiles, co
 }
 
 /* ------------------------------------- sweep with register-pipelined loads */
-/* Operands of one z step of a thread's pair (k_sweep's loads). */
 /* The micSA half-sweep of k_sweep with the loads of z step t+1 issued before
  * the arithmetic and stores of step t, so that a thread always has one step
  * of loads in flight while it computes (see sweep_ahead_block). */
