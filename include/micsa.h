@@ -46,8 +46,8 @@
  *   MICSA_FLOW_HALF=1    half-height dataflow tiles, with a pinned shape
  *   MICSA_FLOW_XS=1      the dataflow sweep takes the remaining x-neighbour word
  *                        from the adjacent lane (warp shuffle), with a pinned shape
- *   MICSA_SWEEP_PF=n     the dataflow sweep requests n demon planes of each tile
- *                        into L2 before its dependency wait
+ *   MICSA_SWEEP_PF=n     with a pinned dataflow shape other than lin: n demon planes
+ *                        of each tile requested into L2 before its dependency wait
  *   MICSA_MULTI_ZC=z     slab depth of the mixed-lattice launch (no timing)
  *   MICSA_MULTI_ITERS=k  iterations per mixed-lattice launch
  *   MICSA_MULTI_RESIDENT=0  small lattices inside the mixed launch too
@@ -232,10 +232,13 @@ int micsa_profile(micsa_ctx *ctx, int64_t n, double *sweep_ms, double *iteration
  * this process (MICSA_TUNE_CACHE=0 times every context instead).  The
  * environment variables MICSA_SWEEP_ZC, MICSA_SWEEP_PD, MICSA_SWEEP_SPLIT,
  * MICSA_SWEEP_OCC, MICSA_SWEEP_TMA, MICSA_SWEEP_ASYNC, MICSA_SWEEP_PIPE,
- * MICSA_SWEEP_FLOW, MICSA_SWEEP_QUAD and MICSA_SWEEP_TILE (=row, or =lin with the dataflow sweep), read by
- * micsa_create, pin the shape and skip the timing (no candidates listed
- * then).  The dataflow sweep is timed for L >= 128 only; MICSA_SWEEP_FLOW=0
- * alone leaves it out everywhere.  The reference has fixed launch geometry
+ * MICSA_SWEEP_FLOW, MICSA_SWEEP_QUAD and MICSA_SWEEP_TILE (=row, or =lin with
+ * the dataflow sweep), read by micsa_create, pin the shape and skip the timing
+ * (no candidates listed then).  The dataflow sweep is timed in tiles of
+ * consecutive units (lin, lin4) for L >= 128 and for smaller contexts that fill
+ * the GPU by themselves; pflow, half-height tiles and the other tile shapes of
+ * flow are only ever pinned.  MICSA_SWEEP_FLOW=0 alone leaves it out
+ * everywhere.  The reference has fixed launch geometry
  * (calculate_blocks, ini.c:580-602). */
 int micsa_tuning_report(const micsa_ctx *ctx, char *buf, size_t n);
 

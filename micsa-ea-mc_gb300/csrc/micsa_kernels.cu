@@ -1069,11 +1069,13 @@ struct micsa_flow_plan {
   int smaj;
 };
 
-/* One tile per block.  Neither DRAM (58% of its peak at L=160) nor the ALU
- * pipe bounds it, but the time a tile spends beside its z loop: the chain of
- * round trips before any warp can load, and the one after the last store
- * before its slot is free again (9600 of a tile's 28600 cycles at L=160, 8
- * planes).  So both are kept short: the ticket is decoded by multiplications
+/* One tile per block.  Neither DRAM (69% of its peak at L=160) nor the ALU
+ * pipe (47%) bounds it, but latency: of the loads in the z loop, and of the time
+ * a tile spends beside it, the chain of round trips before any warp can load
+ * and the one after the last store before its slot is free again (ticket and
+ * first look 2500, dependency wait 1900, release 2200 cycles beside 14100 of
+ * the z loop at 5 planes; 9600 of 28600 at 8 planes before both were kept
+ * short): the ticket is decoded by multiplications
  * instead of divisions; the sample's walk, its run flag and the three slab
  * counters are loaded together, a lane each, by acquire loads that no fence
  * follows; the last warp to finish adds to the slab counter with a release,
@@ -1663,7 +1665,7 @@ __device__ __forceinline__ uint32_t heat_bath_uniforms(uint32_t (&c)[4], uint32_
  * nearly every byte.
  *
  * Bound by latency at the sizes that thermalise (six warps per scheduler at
- * L=64, 64 replicas, 45% of the issue slots): 13.7 us per colour there, 15.9
+ * L=64, 64 replicas, 51% of the issue slots): 13.7 us per colour there, 15.9
  * with the bisection in place and 64-bit site divisions, 14.2 with a thread
  * per 64-bit word (the prologue three times). */
 constexpr int RND_QUEUE = 32 + 128; /* waiting draws per warp: fewer than 32, plus one call's */

@@ -164,19 +164,20 @@ struct slice {
  * Waits are bounded; see halo_lost.
  *
  * What bounds it: with one block per sample the integer ALU pipe (75% busy at
- * L=16, 58 of 86 instructions per pair and half-sweep; 1.2 us of the 15 ...
- * 35 us ends per launch aside, 0.60 us per half-sweep against 0.93 for a
- * kernel that reads every word from shared memory).  With clusters the
- * exchange adds to it: L=32, C=8 runs 0.84 us per half-sweep, 0.60 with the
- * exchange left out (0.19 the demons' pushes and their wait, 0.05 the halos).
- * Tried for the exchange, L=32: whole-plane bulk copies after the barrier
- * 0.93, plain peer stores with a fence and an arrival 0.88, 8-byte pushes of
- * D0 and D1 apart 0.87, the pushes spread over three half-sweeps 0.86; one
- * pair per thread (64 registers) 1.16.  Measured against the half-sweep
- * launches: L=16, one sample x 64 replicas 11.3 -> 3.2 us per iteration;
- * L=24, 2 x 32, nc=5 23.1 -> 5.5; L=32, 24 x 64 65 -> 33 (15 clusters of
- * 221 KB per block fit the GPU at once; 39 in four waves, see
- * resident_rounds). */
+ * L=16, 58 of 86 instructions per pair and half-sweep; the 15 ... 35 us of a
+ * launch's ends aside, 0.59 us per half-sweep against 0.93 for a kernel that
+ * reads every word from shared memory).  With clusters the exchange adds to it
+ * (L=16 by 8 blocks, 0.24 us per half-sweep: the pipe 30% busy).  L=32, C=8 ran
+ * 0.84 us per half-sweep when 0.60 were left without the exchange (0.19 the
+ * demons' pushes and their wait, 0.05 the halos), and runs 0.80 since the waits'
+ * further tries are out of line.  Tried for the exchange, L=32, against 0.84:
+ * whole-plane bulk copies after the barrier 0.93, plain peer stores with a fence
+ * and an arrival 0.88, 8-byte pushes of D0 and D1 apart 0.87, the pushes spread
+ * over three half-sweeps 0.86; one pair per thread (64 registers) 1.16; a state
+ * carried past each wait instead of ending the thread 0.87 to 0.97.  Measured
+ * against the half-sweep launches: L=16, one sample x 64 replicas 11.3 -> 2.9 us
+ * per iteration; L=24, 2 x 32, nc=5 23.1 -> 5.1; L=32, 24 x 64 65 -> 32 (15
+ * clusters of 221 KB per block fit the GPU at once; see resident_rounds). */
 template <int L, int C, int PPT>
 __global__ void __launch_bounds__((rcfg<L, C, PPT>::T), 1)
 k_resident(const micsa_geo g, const slice sl, uint32_t *__restrict__ spin,
@@ -532,10 +533,10 @@ cudaError_t raise_limit(const variant &v, int optin) {
 
 /* Blocks per cluster for a context: the most that still run all of its
  * (sample, word) clusters at once -- more SMs per sample shorten every
- * half-sweep (L=16, one sample: 7.2, 5.5, 4.3 and 3.2 us per iteration with
- * 1, 2, 4 and 8 blocks; L=24: 7.4 and 5.3 with 4 and 8) -- else the fewest,
- * which spend least on the exchange (L=24, 60 samples x 64 replicas: 36 us
- * with 4 blocks, 52 with 8).  pin > 0 asks for that size.
+ * half-sweep (L=16, one sample: 7.1, 5.1, 4.0 and 2.9 us per iteration with
+ * 1, 2, 4 and 8 blocks; L=24 x 2, nc = 5: 7.4 and 5.3 with 4 and 8) -- else the fewest,
+ * which spend least on the exchange (L=24, 60 samples x 64 replicas: 30 us
+ * with 4 blocks; before rounds, 36 with 4 and 52 with 8).  pin > 0 asks for that size.
  *
  * *min_n: the least number of iterations in a call that pays for copying the
  * state in and out.  A launch of v waves of clusters costs about v times
